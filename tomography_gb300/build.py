@@ -31,6 +31,9 @@ SOURCES = [
     "advance_f32_ref.cu",
     "advance_f64.cu",
     "advance_registry.cu",
+    "resident.cu",
+    "resident_f32.cu",
+    "resident_f64.cu",
     "engine.cu",
     "serve.cu",
     "capi.cpp",

@@ -82,7 +82,7 @@ __global__ void bump_kernel(SolveDesc<Real>* descs, int nsolves, int T, int* cou
     SolveDesc<Real>& D = descs[s];
     if (D.active && D.step < D.steps_total) {
         D.step += T;
-        D.parity ^= 1;
+        if (!D.resident) D.parity ^= 1;   // the resident kernel keeps its state in one copy
     }
 }
 

@@ -404,6 +404,7 @@ int unpack_args(const ProblemClass& pc, const double* args, size_t ncand, size_t
     u.ncand = ncand;
     u.upload.assign(ncand * kMaxMat * 3 + ncand * (size_t)K * 6, 0.0);
     u.bbox.assign(ncand * 4, 0);
+    u.mbox.assign(ncand * 4, 0);
     for (size_t c = 0; c < ncand; ++c) {
         const double* a = args + c * nparam;
         double* mp = &u.upload[c * kMaxMat * 3];
@@ -431,18 +432,21 @@ int unpack_args(const ProblemClass& pc, const double* args, size_t ncand, size_t
             const int r = (int)std::ceil(s.breast_radius / s.dx) + 2;
             bb[0] = std::max(1, s.nx / 2 - r); bb[1] = std::min(s.nx - 1, s.nx / 2 + r);
             bb[2] = std::max(1, s.ny / 2 - r); bb[3] = std::min(s.ny - 1, s.ny / 2 + r);
+            std::copy(bb, bb + 4, &u.mbox[c * 4]);
             continue;
         }
         mp[0] = s.bg_eps_inf; mp[1] = s.bg_del_eps; mp[2] = s.bg_sigma;
         mp[3] = s.disc_eps_inf; mp[4] = s.disc_del_eps; mp[5] = s.disc_sigma;
         double* el = &u.upload[ncand * kMaxMat * 3 + c * (size_t)K * 6];
-        double xlo = 1e30, xhi = -1e30, ylo = 1e30, yhi = -1e30;
-        auto grow = [&](double cx, double cy, double r) {
-            xlo = std::min(xlo, cx - r); xhi = std::max(xhi, cx + r);
-            ylo = std::min(ylo, cy - r); yhi = std::max(yhi, cy + r);
+        // extents (x low, x high, y low, y high) of the dispersive shapes and of all shapes
+        double disp[4] = {1e30, -1e30, 1e30, -1e30}, any[4] = {1e30, -1e30, 1e30, -1e30};
+        auto grow = [](double* v, double cx, double cy, double r) {
+            v[0] = std::min(v[0], cx - r); v[1] = std::max(v[1], cx + r);
+            v[2] = std::min(v[2], cy - r); v[3] = std::max(v[3], cy + r);
         };
         bool everywhere = s.bg_del_eps != 0;
-        if (s.disc_radius > 0 && s.disc_del_eps != 0) grow(0, 0, s.disc_radius);
+        if (s.disc_radius > 0) grow(any, 0, 0, s.disc_radius);
+        if (s.disc_radius > 0 && s.disc_del_eps != 0) grow(disp, 0, 0, s.disc_radius);
         for (int k = 0; k < K; ++k) {
             const double* e = a + 8 * k;
             if (!(e[2] > 0) || !(e[3] > 0)) return fail(TOMO_EINVAL, "ellipse semi-axes must be positive");
@@ -456,7 +460,8 @@ int unpack_args(const ProblemClass& pc, const double* args, size_t ncand, size_t
             mp[3 * (2 + k) + 0] = e[5];
             mp[3 * (2 + k) + 1] = e[6];
             mp[3 * (2 + k) + 2] = e[7];
-            if (e[6] != 0) grow(e[0], e[1], std::max(e[2], e[3]));
+            grow(any, e[0], e[1], std::max(e[2], e[3]));
+            if (e[6] != 0) grow(disp, e[0], e[1], std::max(e[2], e[3]));
         }
         // Jp can be non-zero only where del_eps != 0: conservative cell box
         auto cell = [&](double v, int n, bool up) {
@@ -465,12 +470,14 @@ int unpack_args(const ProblemClass& pc, const double* args, size_t ncand, size_t
             r = std::max(1.0, std::min((double)(n - 1), r));
             return (int)r;
         };
+        auto box = [&](const double* v, int* o) {
+            if (v[1] < v[0]) { o[0] = 1; o[1] = 0; o[2] = 1; o[3] = 0; return; }
+            o[0] = cell(v[0], s.nx, false); o[1] = cell(v[1], s.nx, true);
+            o[2] = cell(v[2], s.ny, false); o[3] = cell(v[3], s.ny, true);
+        };
+        box(disp, bb);
+        box(any, &u.mbox[c * 4]);
         if (everywhere) { bb[0] = 1; bb[1] = s.nx - 1; bb[2] = 1; bb[3] = s.ny - 1; }
-        else if (xhi < xlo) { bb[0] = 1; bb[1] = 0; bb[2] = 1; bb[3] = 0; }
-        else {
-            bb[0] = cell(xlo, s.nx, false); bb[1] = cell(xhi, s.nx, true);
-            bb[2] = cell(ylo, s.ny, false); bb[3] = cell(yhi, s.ny, true);
-        }
     }
     return TOMO_OK;
 }
@@ -512,6 +519,96 @@ int EngineT<Real>::init(const ProblemClass& pc) {
     if (c.empty())
         return fail(TOMO_EINVAL, "unsupported (steps_per_launch, cols_per_lane) pair for this mode and precision");
     blk_ = c.front();   // until the first batch is tuned
+    if (auto_T_ && auto_cols_ && auto_minb_ && !pc.spec.plain)
+        for (int blocks : {16, 8, 4}) {
+            ResidentPlan p;
+            if (resident_plan<Real>(cd_.pc, cd_.lay, blocks, p)) plans_.push_back(p);
+        }
+    plan_batch_.resize(plans_.size());
+    return TOMO_OK;
+}
+
+// Fills and uploads the descriptors of the current batch at step 0.
+template <typename Real>
+int EngineT<Real>::upload_descs(size_t ncand) {
+    const ProblemClass& pc = cd_.pc;
+    const int nsolves = nsolves_;
+    h_descs_.resize(nsolves);
+    fill_descs<Real>(cd_, up_, d_state_.as<Real>(), d_mats_.as<uint8_t>(), d_tabs_.as<Real>(), h_descs_.data());
+    if (pc.extra)
+        h_descs_[nsolves - 1] =
+            incident_desc<Real>(cd_, d_state_.as<Real>() + (size_t)(nsolves - 1) * cd_.lay.per_solve);
+    if (blk_.blocks > 0) 
+        make_resident<Real>(pc, cd_.lay, plans_[plan_at_], plan_batch_[plan_at_], up_, h_descs_.data(), nsolves);
+    else if (!pc.spec.plain)   // the time-loop graph runs one DFT pass per group of launches
+        for (SolveDesc<Real>& D : h_descs_) D.stage_group = stage_group_for(blk_.T);
+    CUDA_TRY(cudaMemcpyAsync(d_descs_.p, h_descs_.data(), sizeof(SolveDesc<Real>) * nsolves, cudaMemcpyHostToDevice,
+                             stream_));
+    (void)ncand;
+    return TOMO_OK;
+}
+
+// Times every resident plan that fits the batch (the time of a launch of 40
+// steps less that of one of 8: the slabs' loading and storing cancels) and
+// keeps the fastest; blk_ and plan_ are set.
+template <typename Real>
+int EngineT<Real>::autotune_resident(size_t ncand) {
+    constexpr int kShort = 8, kLong = 40;
+    const ProblemClass& pc = cd_.pc;
+    const int mode = advance_mode(pc.spec), key = (int)ncand * pc.n_exc;
+    auto use = [&](size_t i) {
+        plan_at_ = i;
+        blk_ = Blocking{std::min(plans_[i].levels, pc.S), Quad<Real>::N, 1, plans_[i].blocks};
+    };
+    std::vector<size_t> fit;
+    for (size_t i = 0; i < plans_.size(); ++i)
+        if (plan_batch_[i].fits) fit.push_back(i);
+    const auto known = tuned_resident_.find(key);
+    if (known != tuned_resident_.end())
+        for (size_t i : fit)
+            if (plans_[i].blocks == known->second.blocks) {
+                use(i);
+                return TOMO_OK;
+            }
+    use(fit.front());
+    if (known != tuned_resident_.end()) return TOMO_OK;   // the tuned one does not fit this batch
+    if (fit.size() > 1 && pc.S >= kShort + kLong) {
+        TOMO_TRY(ensure_batch((int)ncand));
+        const int nsolves = nsolves_;
+        TOMO_TRY(d_upload_.ensure(sizeof(double) * up_.upload.size()));
+        int64_t kernels = 0, h2d = 0;
+        TOMO_TRY(setup_materials<Real>(cd_, up_, d_upload_.as<double>(), d_mats_.as<uint8_t>(), d_tabs_.as<Real>(),
+                                       stream_, &kernels, &h2d));
+        CUDA_TRY(cudaMemsetAsync(d_state_.p, 0, (size_t)nsolves * cd_.lay.per_solve * sizeof(Real), stream_));
+        double best = 1e300;
+        size_t besti = fit.front();
+        for (size_t i : fit) {
+            use(i);
+            TOMO_TRY(upload_descs(ncand));
+            int clusters = 0;
+            TOMO_TRY(resident_clusters<Real>(plans_[plan_at_], plan_batch_[plan_at_], mode, &clusters));
+            TOMO_TRY(launch_resident<Real>(plans_[plan_at_], plan_batch_[plan_at_], mode, clusters, d_descs_.as<SolveDesc<Real>>(), nsolves, 1,
+                                           d_counter_.as<int>() + 1, stream_));
+            float ms[2] = {0, 0};
+            for (int l = 0; l < 2; ++l) {
+                CUDA_TRY(cudaEventRecord(ev_[1], stream_));
+                TOMO_TRY(launch_resident<Real>(plans_[plan_at_], plan_batch_[plan_at_], mode, clusters, d_descs_.as<SolveDesc<Real>>(), nsolves,
+                                               std::min(l ? kLong : kShort, plans_[i].levels), d_counter_.as<int>() + 1,
+                                               stream_));
+                CUDA_TRY(cudaEventRecord(ev_[2], stream_));
+                CUDA_TRY(cudaStreamSynchronize(stream_));
+                CUDA_TRY(cudaEventElapsedTime(&ms[l], ev_[1], ev_[2]));
+                stats_.tune_ms += ms[l];
+            }
+            ++stats_.tuned_configs;
+            if (ms[1] - ms[0] < best) {
+                best = ms[1] - ms[0];
+                besti = i;
+            }
+        }
+        use(besti);
+    }
+    tuned_resident_[key] = blk_;
     return TOMO_OK;
 }
 
@@ -571,11 +668,11 @@ int EngineT<Real>::autotune(size_t ncand) {
         TOMO_TRY(advance_grid<Real>(c, mode, (int)items.size(), num_sms_, &blocks, &smem));
         const int L = std::max(2, kTuneSteps / c.T);
         launch_advance<Real>(c, mode, blocks, smem, d_descs_.as<SolveDesc<Real>>(), d_tune_items_.as<WorkItem>(),
-                             (int)items.size(), nsolves, d_counter_.as<int>(), dft_contour(pc), stream_);
+                             (int)items.size(), nsolves, d_counter_.as<int>(), dft_contour(pc), std::max(1, pc.nfreq), stream_);
         CUDA_TRY(cudaEventRecord(ev_[1], stream_));
         for (int l = 0; l < L; ++l)
             launch_advance<Real>(c, mode, blocks, smem, d_descs_.as<SolveDesc<Real>>(), d_tune_items_.as<WorkItem>(),
-                                 (int)items.size(), nsolves, d_counter_.as<int>(), dft_contour(pc), stream_);
+                                 (int)items.size(), nsolves, d_counter_.as<int>(), dft_contour(pc), std::max(1, pc.nfreq), stream_);
         CUDA_TRY(cudaEventRecord(ev_[2], stream_));
         CUDA_TRY(cudaStreamSynchronize(stream_));
         CUDA_TRY(cudaGetLastError());
@@ -641,6 +738,15 @@ int EngineT<Real>::ensure_batch(int ncand) {
         }
         cap_cand_ = ncand;
     }
+    if (blk_.blocks > 0) {   // the resident kernel has no work items
+        if (nsolves != nsolves_ || ncand != cur_cand_) {
+            invalidate_graph();
+            items_blk_ = Blocking{-1, -1, -1};
+        }
+        nsolves_ = nsolves;
+        cur_cand_ = ncand;
+        return TOMO_OK;
+    }
     std::vector<WorkItem> items;
     const int nseg = choose_segments(
         (long)nsolves * items_per_solve(pc.nx, pc.ny, pc.nc, item_face_distance(pc), blk_.T, blk_.cols), pc.ny,
@@ -663,26 +769,44 @@ int EngineT<Real>::ensure_batch(int ncand) {
 
 template <typename Real>
 int EngineT<Real>::build_graph(int nlaunch) {
-    if (graph_exec_ && graph_cand_ == cur_cand_ && graph_blk_ == blk_ && graph_launches_ == nlaunch)
+    const bool resident = blk_.blocks > 0;
+    if (graph_exec_ && graph_cand_ == cur_cand_ && graph_blk_ == blk_ && graph_launches_ == nlaunch &&
+        (!resident || (graph_smem_ == plan_batch_[plan_at_].smem && graph_warps_ == plan_batch_[plan_at_].warps)))
         return TOMO_OK;
     invalidate_graph();
-    int blocks = 0;
+    int blocks = 0, clusters = 0;
     size_t smem = 0;
-    TOMO_TRY(advance_grid<Real>(blk_, advance_mode(cd_.pc.spec), nitems_, num_sms_, &blocks, &smem));
+    const int mode = advance_mode(cd_.pc.spec);
+    if (resident) TOMO_TRY(resident_clusters<Real>(plans_[plan_at_], plan_batch_[plan_at_], mode, &clusters));
+    else TOMO_TRY(advance_grid<Real>(blk_, mode, nitems_, num_sms_, &blocks, &smem));
     cudaGraph_t graph;
     CUDA_TRY(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
     // one DFT pass per group of stage_group launches (and after the last launch):
     // it sums the group's steps in time order, as one pass per launch would
     const int group = stage_group_for(blk_.T), S = cd_.pc.S, T = blk_.T;
-    for (int l = 0; l < nlaunch; ++l) {
+    int rc = TOMO_OK;
+    for (int l = 0; resident && l < nlaunch && rc == TOMO_OK; ++l) {
+        rc = launch_resident<Real>(plans_[plan_at_], plan_batch_[plan_at_], mode, clusters, d_descs_.as<SolveDesc<Real>>(), nsolves_, T,
+                                   d_counter_.as<int>() + 1, stream_);
+        if (dft_contour(cd_.pc) > 0)
+            launch_dft<Real>(d_descs_.as<SolveDesc<Real>>(), nsolves_, dft_contour(cd_.pc), cd_.pc.nfreq, T, l * T,
+                             std::min(T, S - l * T), stream_);
+        bump_kernel<Real><<<(nsolves_ + 127) / 128, 128, 0, stream_>>>(d_descs_.as<SolveDesc<Real>>(), nsolves_, T,
+                                                                       d_counter_.as<int>());
+    }
+    for (int l = 0; !resident && l < nlaunch; ++l) {
         const bool last_of_group = (l + 1) % group == 0 || l == nlaunch - 1;
         const int n0 = (l - l % group) * T;
         const int nlev = last_of_group ? std::min((l + 1) * T, S) - n0 : 0;
-        launch_advance<Real>(blk_, advance_mode(cd_.pc.spec), blocks, smem, d_descs_.as<SolveDesc<Real>>(),
+        launch_advance<Real>(blk_, mode, blocks, smem, d_descs_.as<SolveDesc<Real>>(),
                              d_items_.as<WorkItem>(), nitems_, nsolves_, d_counter_.as<int>(), dft_contour(cd_.pc),
-                             stream_, n0, nlev);
+                             std::max(1, cd_.pc.nfreq), stream_, n0, nlev);
     }
     cudaError_t ce = cudaStreamEndCapture(stream_, &graph);
+    if (rc) {
+        if (ce == cudaSuccess) cudaGraphDestroy(graph);
+        return rc;
+    }
     if (ce != cudaSuccess) return fail(TOMO_ECUDA, std::string("graph capture: ") + cudaGetErrorString(ce));
     ce = cudaGraphInstantiate(&graph_exec_, graph, 0);
     cudaGraphDestroy(graph);
@@ -691,6 +815,10 @@ int EngineT<Real>::build_graph(int nlaunch) {
         return fail(TOMO_ECUDA, std::string("graph instantiate: ") + cudaGetErrorString(ce));
     }
     graph_cand_ = cur_cand_; graph_blk_ = blk_; graph_launches_ = nlaunch; graph_blocks_ = blocks;
+    if (resident) {
+        graph_smem_ = plan_batch_[plan_at_].smem;
+        graph_warps_ = plan_batch_[plan_at_].warps;
+    }
     return TOMO_OK;
 }
 
@@ -703,7 +831,14 @@ int EngineT<Real>::forward(const double* args, size_t ncand, size_t nparam, cons
     TOMO_TRY(unpack_args(pc, args, ncand, nparam, up_));
     stats_.tune_ms = 0;
     stats_.tuned_configs = 0;
-    if ((auto_T_ || auto_cols_ || auto_minb_) && !s.plain) {
+    bool fits = false;
+    for (size_t i = 0; i < plans_.size(); ++i) {
+        resident_batch<Real>(pc, plans_[i], up_, plan_batch_[i]);
+        fits |= plan_batch_[i].fits;
+    }
+    if (fits) {
+        TOMO_TRY(autotune_resident(ncand));
+    } else if ((auto_T_ || auto_cols_ || auto_minb_) && !s.plain) {
         auto it = tuned_.find((int)ncand * pc.n_exc);
         if (it != tuned_.end()) {
             blk_ = it->second;
@@ -723,13 +858,7 @@ int EngineT<Real>::forward(const double* args, size_t ncand, size_t nparam, cons
     TOMO_TRY(setup_materials<Real>(cd_, up_, d_upload_.as<double>(), d_mats_.as<uint8_t>(), d_tabs_.as<Real>(), stream_,
                                    &kernels, nullptr));
     CUDA_TRY(cudaMemsetAsync(d_state_.p, 0, (size_t)nsolves * cd_.lay.per_solve * sizeof(Real), stream_));
-    h_descs_.resize(nsolves);
-    fill_descs<Real>(cd_, up_, d_state_.as<Real>(), d_mats_.as<uint8_t>(), d_tabs_.as<Real>(), h_descs_.data());
-    if (pc.extra) h_descs_[nsolves - 1] = incident_desc<Real>(cd_, d_state_.as<Real>() + (size_t)(nsolves - 1) * cd_.lay.per_solve);
-    if (!s.plain)   // the time-loop graph runs one DFT pass per group of launches
-        for (SolveDesc<Real>& D : h_descs_) D.stage_group = stage_group_for(blk_.T);
-    CUDA_TRY(cudaMemcpyAsync(d_descs_.p, h_descs_.data(), sizeof(SolveDesc<Real>) * nsolves, cudaMemcpyHostToDevice,
-                             stream_));
+    TOMO_TRY(upload_descs(ncand));
     h2d += sizeof(SolveDesc<Real>) * nsolves;
 
     // time loop: ceil(S/T) advance launches, each followed by the running DFT and
@@ -752,7 +881,8 @@ int EngineT<Real>::forward(const double* args, size_t ncand, size_t nparam, cons
         CUDA_TRY(cudaGraphLaunch(graph_exec_, stream_));
         CUDA_TRY(cudaEventRecord(ev_[2], stream_));
         const int group = stage_group_for(blk_.T);
-        kernels += 2 * (int64_t)nlaunch + (dft_contour(pc) > 0 ? (nlaunch + group - 1) / group : 0);
+        const int passes = blk_.blocks > 0 ? nlaunch : (nlaunch + group - 1) / group;
+        kernels += 2 * (int64_t)nlaunch + (dft_contour(pc) > 0 ? passes : 0);
     }
 
     CUDA_TRY(cudaMemsetAsync(d_flag_.p, 0, sizeof(int) * 4, stream_));
@@ -794,7 +924,9 @@ int EngineT<Real>::forward(const double* args, size_t ncand, size_t nparam, cons
         }
     }
     CUDA_TRY(cudaEventRecord(ev_[3], stream_));
-    int flag = 0;
+    int flag = 0, lost = 0;
+    if (blk_.blocks > 0)
+        CUDA_TRY(cudaMemcpyAsync(&lost, d_counter_.as<int>() + 1, sizeof(int), cudaMemcpyDeviceToHost, stream_));
     if (want_fit) {
         CUDA_TRY(cudaMemcpyAsync(out->fitness, d_fit_.p, sizeof(double) * ncand, cudaMemcpyDeviceToHost, stream_));
         CUDA_TRY(cudaMemcpyAsync(&flag, d_flag_.p, sizeof(int), cudaMemcpyDeviceToHost, stream_));
@@ -802,6 +934,10 @@ int EngineT<Real>::forward(const double* args, size_t ncand, size_t nparam, cons
     }
     CUDA_TRY(cudaStreamSynchronize(stream_));
     CUDA_TRY(cudaGetLastError());
+    if (lost) {
+        CUDA_TRY(cudaMemset(d_counter_.as<int>() + 1, 0, sizeof(int)));
+        return fail(TOMO_ECUDA, "internal error: a halo row of the resident kernel did not arrive");
+    }
     float adv = 0, tot = 0;
     CUDA_TRY(cudaEventElapsedTime(&adv, ev_[1], ev_[2]));
     CUDA_TRY(cudaEventElapsedTime(&tot, ev_[0], ev_[3]));
@@ -810,7 +946,8 @@ int EngineT<Real>::forward(const double* args, size_t ncand, size_t nparam, cons
     stats_.cell_updates = (double)nsolves * (double)s.nx * (double)s.ny * (double)pc.S;
     stats_.launches = s.plain ? (int64_t)pc.S * nsolves : nlaunch;
     have_batch_ = true;
-    last_parity_ = s.plain ? 0 : (nlaunch & 1);   // the plain path updates copy 0 in place
+    // the plain path and the resident kernel update copy 0 in place
+    last_parity_ = s.plain || blk_.blocks > 0 ? 0 : (nlaunch & 1);
     stats_.kernels = kernels;
     stats_.steps_per_launch = blk_.T;
     stats_.cols_per_lane = blk_.cols;

@@ -18,6 +18,7 @@
 #include "aux_kernels.cuh"
 #include "engine.h"
 #include "fdtd_advance.cuh"
+#include "fdtd_resident.cuh"
 #include "solve_desc.h"
 
 #define CUDA_TRY(expr)                                                                                      \
@@ -102,15 +103,20 @@ SolveLayout solve_layout(const ProblemClass& pc, size_t real_bytes);
 struct Unpacked {
     std::vector<double> upload;   // [ncand][kMaxMat][3] then [ncand][K][6]
     std::vector<int> bbox;        // [ncand][4] dispersive box (x0, x1, y0, y1)
+    std::vector<int> mbox;        // [ncand][4] box of every cell that is not background
     size_t ncand = 0;
 };
 int unpack_args(const ProblemClass& pc, const double* args, size_t ncand, size_t nparam, Unpacked& u);
 
 // Blocking of the advance kernel: time steps per launch, columns per lane, and
-// the minimum resident blocks per SM its registers were allocated for.
+// the minimum resident blocks per SM its registers were allocated for.  With
+// blocks > 0 it is the resident kernel instead: T steps per launch, clusters of
+// that many blocks per solve.
 struct Blocking {
-    int T = 1, cols = 1, minb = 2;
-    bool operator==(const Blocking& o) const { return T == o.T && cols == o.cols && minb == o.minb; }
+    int T = 1, cols = 1, minb = 2, blocks = 0;
+    bool operator==(const Blocking& o) const {
+        return T == o.T && cols == o.cols && minb == o.minb && blocks == o.blocks;
+    }
     bool operator!=(const Blocking& o) const { return !(*this == o); }
 };
 
@@ -401,6 +407,40 @@ std::vector<Blocking> tune_candidates(int mode, int fixT, int fixCols, int fixMi
     return out;
 }
 
+// ------------------------------------------------------------ resident kernel
+constexpr size_t kSmemPerBlock = 227 * 1024;
+constexpr int kResidentSteps = 512;   // most time steps of one resident launch
+
+// How a problem class runs on clusters of `blocks` blocks (fdtd_resident.cuh).
+struct ResidentPlan {
+    int blocks = 0, passes = 0, levels = 0;
+};
+// A batch on a plan: every candidate's slabs, and what a launch needs.
+struct ResidentBatch {
+    bool fits = false;
+    int warps = 0;             // per block
+    size_t smem = 0;           // per block
+    std::vector<int> ys;       // [ncand (+ 1)][blocks + 1]: first row of each slab, then ny
+};
+// false: the class does not fit the resident kernel with that many blocks.
+template <typename Real>
+bool resident_plan(const ProblemClass& pc, const SolveLayout& lay, int blocks, ResidentPlan& p);
+// Cuts the candidates' rows into slabs; the batch fits when its shared memory does.
+template <typename Real>
+void resident_batch(const ProblemClass& pc, const ResidentPlan& p, const Unpacked& u, ResidentBatch& b);
+// Turns filled descriptors into resident ones (fields in copy 0, the second
+// copies' memory as the staging buffer).  A descriptor past the candidates (the
+// incident grid) has no materials.
+template <typename Real>
+void make_resident(const ProblemClass& pc, const SolveLayout& lay, const ResidentPlan& p, const ResidentBatch& b,
+                   const Unpacked& u, SolveDesc<Real>* descs, int nsolves);
+// Clusters of the batch that run at once, and one launch of nsteps steps.
+template <typename Real>
+int resident_clusters(const ResidentPlan& p, const ResidentBatch& b, int mode, int* clusters);
+template <typename Real>
+int launch_resident(const ResidentPlan& p, const ResidentBatch& b, int mode, int clusters, const SolveDesc<Real>* descs,
+                    int nsolves, int nsteps, int* error, cudaStream_t st);
+
 // One time step of one solve on the plain path (H, E and DFT kernels; the DFT
 // kernel only when n_contour > 0).  Returns the number of kernels launched.
 template <typename Real>
@@ -410,20 +450,26 @@ int launch_plain_step(int mode, const SolveDesc<Real>* d, int n, int nx, int ny,
 // engine's descriptors at blocking T).
 inline int stage_group_for(int T) { return std::max(1, kStageLevels / std::max(T, 1)); }
 
+template <typename Real>
+void launch_dft(const SolveDesc<Real>* descs, int nsolves, int cmax, int fmax, int T, int n0, int nlev,
+                cudaStream_t st) {
+    dft_accumulate_kernel<Real><<<dim3(nsolves * fmax, (cmax + 127) / 128), 128, 0, st>>>(descs, T, fmax, n0, nlev);
+}
+
 // One advance launch (T steps of every listed solve), then -- when cmax, the
 // largest contour among the solves, is positive and dft_nlev is not 0 -- the
-// running DFT of the staged contour samples (dft_n0 < 0: this launch's levels;
+// running DFT over at most fmax frequencies of the staged contour samples (dft_n0 < 0: this launch's levels;
 // else steps dft_n0 .. dft_n0 + dft_nlev - 1), then the progress bump.
 // Returns the number of kernels.
 template <typename Real>
 int launch_advance(const Blocking& b, int mode, int blocks, size_t smem, const SolveDesc<Real>* descs,
-                   const WorkItem* items, int nitems, int nsolves, int* counter, int cmax, cudaStream_t st,
+                   const WorkItem* items, int nitems, int nsolves, int* counter, int cmax, int fmax, cudaStream_t st,
                    int dft_n0 = -1, int dft_nlev = -1) {
     AdvanceFn<Real> fn = advance_kernel_for<Real>(b, mode);
     fn<<<blocks, 128, smem, st>>>(descs, items, nitems, counter);
     const bool dft = cmax > 0 && dft_nlev != 0;
     if (dft)
-        dft_accumulate_kernel<Real><<<dim3(nsolves, (cmax + 127) / 128), 128, 0, st>>>(descs, b.T, dft_n0, dft_nlev);
+        launch_dft<Real>(descs, nsolves, cmax, fmax, b.T, dft_n0, dft_nlev, st);
     bump_kernel<Real><<<(nsolves + 127) / 128, 128, 0, st>>>(const_cast<SolveDesc<Real>*>(descs), nsolves, b.T,
                                                             counter);
     return dft ? 3 : 2;
@@ -576,6 +622,8 @@ class EngineT : public EngineBase {
     int ensure_batch(int ncand);
     int build_graph(int nlaunch);
     int autotune(size_t ncand);
+    int autotune_resident(size_t ncand);
+    int upload_descs(size_t ncand);
     void invalidate_graph() {
         if (graph_exec_) cudaGraphExecDestroy(graph_exec_);
         graph_exec_ = nullptr;
@@ -594,6 +642,12 @@ class EngineT : public EngineBase {
     bool auto_T_ = false, auto_cols_ = false, auto_minb_ = false;   // tuned per batch size on first use
     int fix_T_ = 0, fix_cols_ = 0, fix_minb_ = 0;  // dimensions fixed by the spec or the environment
     std::map<int, Blocking> tuned_;                // solves per batch -> blocking
+    std::map<int, Blocking> tuned_resident_;       // the same among the resident plans
+    std::vector<ResidentPlan> plans_;              // resident plans of the class, most blocks first
+    std::vector<ResidentBatch> plan_batch_;        // the current batch on each
+    size_t plan_at_ = 0;                           // the one of blk_ when blk_.blocks > 0
+    size_t graph_smem_ = 0;
+    int graph_warps_ = 0;
     Blocking items_blk_{-1, -1, -1};               // blocking the uploaded work items were cut for
     DevBuf d_tune_items_;
     uint64_t budget_ = (uint64_t)150 << 30;

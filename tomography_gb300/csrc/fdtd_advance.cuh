@@ -167,7 +167,7 @@ __device__ __forceinline__ void dft_update(Real* acc, const Real* ph, int nfreq,
 }
 
 // Running DFT of the NTFF contour (FDTD_GPU.cu:231-280) for the time steps the
-// last advance launch computed: one thread per (solve, contour point) adds the
+// last advance launch computed: one thread per (solve, frequency, contour point) adds the
 // staged (h, e) samples of the launch's levels in time order, with the same
 // compensated sums as one update per step.  Runs between the advance launch
 // and the progress bump (which moves `step`).
@@ -209,31 +209,32 @@ constexpr int kStageLevels = 8;
 
 template <typename Real>
 __global__ void __launch_bounds__(128) dft_accumulate_kernel(const SolveDesc<Real>* __restrict__ descs, int T,
-                                                             int n0_group, int nlev) {
-    const SolveDesc<Real>& D = descs[blockIdx.x];
+                                                             int fmax, int n0_group, int nlev) {
+    const SolveDesc<Real>& D = descs[blockIdx.x / fmax];
+    const int f = blockIdx.x % fmax;
     const int c = blockIdx.y * blockDim.x + threadIdx.x;
     const int C = D.n_contour, nfreq = D.nfreq;
-    if (!D.active || nfreq <= 0 || c >= C) return;
+    if (!D.active || f >= nfreq || c >= C) return;
     const int n0 = n0_group >= 0 ? n0_group : D.step;
     const int nsteps = min(n0_group >= 0 ? nlev : T, D.steps_total - n0);
-    for (int f = 0; f < nfreq; ++f) {
-        Real* a = D.acc + ((size_t)f * C + c) * 8;
-        Real j[4], mm[4];   // J: sum re, sum im, comp re, comp im; M likewise
-        Vec4<Real>::load(a, j);
-        Vec4<Real>::load(a + 4, mm);
-        for (int k = 0; k < nsteps; ++k) {
-            Real p[4];
-            Vec4<Real>::load(D.phasor + ((size_t)(n0 + k) * nfreq + f) * 4, p);
-            const Real* sp = D.stage + ((size_t)k * C + c) * 2;
-            const Real h = sp[0], e = sp[1];
-            acc_add(j[0], j[2], Op<Real>::mul(h, p[0]));
-            acc_add(j[1], j[3], Op<Real>::mul(h, p[1]));
-            acc_add(mm[0], mm[2], Op<Real>::mul(e, p[2]));
-            acc_add(mm[1], mm[3], Op<Real>::mul(e, p[3]));
-        }
-        Vec4<Real>::store(a, j);
-        Vec4<Real>::store(a + 4, mm);
+    Real* a = D.acc + ((size_t)f * C + c) * 8;
+    Real j[4], mm[4];   // J: sum re, sum im, comp re, comp im; M likewise
+    Vec4<Real>::load(a, j);
+    Vec4<Real>::load(a + 4, mm);
+    const Real* sp = D.stage + (size_t)c * 2;
+    const Real* pp = D.phasor + ((size_t)n0 * nfreq + f) * 4;
+#pragma unroll 4
+    for (int k = 0; k < nsteps; ++k) {
+        Real p[4];
+        Vec4<Real>::load(pp + (size_t)k * nfreq * 4, p);
+        const Real h = sp[(size_t)k * C * 2], e = sp[(size_t)k * C * 2 + 1];
+        acc_add(j[0], j[2], Op<Real>::mul(h, p[0]));
+        acc_add(j[1], j[3], Op<Real>::mul(h, p[1]));
+        acc_add(mm[0], mm[2], Op<Real>::mul(e, p[2]));
+        acc_add(mm[1], mm[3], Op<Real>::mul(e, p[3]));
     }
+    Vec4<Real>::store(a, j);
+    Vec4<Real>::store(a + 4, mm);
 }
 
 // Two adjacent values as one streaming store (aligned to twice the element size).

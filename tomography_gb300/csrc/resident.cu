@@ -1,0 +1,186 @@
+// Host side of the resident kernel: which problems fit it, how the rows are cut
+// into slabs, and the cluster launch.
+#include "engine_impl.cuh"
+
+namespace tomo {
+
+template <typename Real>
+bool resident_plan(const ProblemClass& pc, const SolveLayout& lay, int blocks, ResidentPlan& p) {
+    const tomo_spec& s = pc.spec;
+    const int rows = pc.ny - 1;
+    // the edge pass holds the PEC columns and the x-CPML; background cells carry no Debye current
+    if (pc.nc > kEdge - 1 || pc.nx < 3 * kEdge || blocks > kMaxSlabs || rows < 4 * blocks) return false;
+    if (s.mode == TOMO_MODE_BREAST && s.bg_del_eps != 0) return false;
+    if (pc.nfreq > 0 && s.nf2ff_d < pc.nc) return false;   // Hy of the NTFF face columns has no x-CPML
+    if (s.mode != TOMO_MODE_BREAST) {
+        // the reference's strips replace the whole update: patches stay clear of them
+        const int r = (int)std::ceil(s.breast_radius / s.dx) + 2, clear = std::max(kEdge, pc.nc + 1);
+        if (pc.nx / 2 - r < clear || pc.nx / 2 + r > pc.nx - clear - 1) return false;
+    }
+    const int right = resident_right<Real>(pc.nx), width = 32 * Quad<Real>::N;
+    if (right > pc.nx - std::max(pc.nc, 1)) return false;   // the x-CPML and PEC columns belong to the edge pass
+    p.blocks = blocks;
+    p.passes = (right - kEdge + width - 1) / width;
+    if (!resident_kernel_for<Real>(p.passes, advance_mode(s))) return false;
+    if (rows > kRows * resident_warps(p.passes) * blocks) return false;
+    // staging levels in the memory of the second field copies
+    p.levels = kResidentSteps;
+    if (pc.nfreq > 0)
+        p.levels = (int)std::min<size_t>(kResidentSteps, (4 * lay.field_elems - kPadLeft) / (2 * (size_t)pc.C));
+    return p.levels >= 1;
+}
+
+// Cuts rows 1 .. ny-1 into slabs of about equal cost: the least cost of the
+// dearest slab, by bisection over a greedy cut.  box: the candidate's materials.
+template <typename Real>
+static bool cut_slabs(const ProblemClass& pc, const ResidentPlan& p, const int* box, std::vector<double>& cost, int* ys) {
+    const int most = kRows * resident_warps(p.passes), width = 32 * Quad<Real>::N;
+    // cost of a row, from the passes' measured times: a plain pass 0.14, one with
+    // materials or y-CPML 0.42, the rest of a row 0.6
+    int mats = 0;
+    for (int c = 0; c < p.passes; ++c)
+        mats += box[0] < kEdge + (c + 1) * width && box[1] >= kEdge + c * width;
+    cost.assign(pc.ny, 0.0);
+    double total = 0;
+    for (int m = 1; m < pc.ny; ++m) {
+        const bool strip = m <= pc.nc || m >= pc.ny - pc.nc, mat = m >= box[2] && m <= box[3];
+        cost[m] = strip ? 0.8 + 0.42 * p.passes : 0.6 + 0.14 * p.passes + (mat ? 0.28 * mats : 0.0);
+        total += cost[m];
+    }
+    // a slab does not end at a horizontal NTFF face: its sample takes Ez of the row above
+    const int face0 = pc.nfreq > 0 ? pc.spec.nf2ff_d : -1, face1 = pc.nfreq > 0 ? pc.ny - pc.spec.nf2ff_d - 1 : -1;
+    auto cut = [&](double limit) {
+        int m = 1;
+        for (int b = 0; b < p.blocks; ++b) {
+            ys[b] = m;
+            const int left = p.blocks - 1 - b;
+            double c = 0;
+            int n = 0;
+            while (m < pc.ny && pc.ny - m > 2 * left && n < most && (n < 2 || c + cost[m] <= limit)) {
+                c += cost[m];
+                ++m;
+                ++n;
+            }
+            if ((m - 1 == face0 || m - 1 == face1) && left > 0) {
+                if (n > 2) --m;
+                else return false;
+            }
+        }
+        ys[p.blocks] = pc.ny;
+        return m == pc.ny;
+    };
+    double lo = 0, hi = 4 * total / p.blocks;
+    if (!cut(hi)) return false;
+    for (int i = 0; i < 12; ++i) {
+        const double mid = 0.5 * (lo + hi);
+        if (cut(mid)) hi = mid;
+        else lo = mid;
+    }
+    if (!cut(hi)) return false;
+    for (int b = 0; b < p.blocks; ++b)
+        if (ys[b + 1] - ys[b] < 2) return false;
+    return true;
+}
+
+template <typename Real>
+void resident_batch(const ProblemClass& pc, const ResidentPlan& p, const Unpacked& u, ResidentBatch& b) {
+    const bool ref = pc.spec.mode != TOMO_MODE_BREAST;
+    const int nb = p.blocks + 1, d = pc.nfreq > 0 ? pc.spec.nf2ff_d : -1, none[4] = {1, 0, 1, 0};
+    const size_t n = u.ncand + pc.extra;
+    b.fits = false;
+    b.warps = 0;
+    b.smem = 0;
+    b.ys.resize(n * nb);
+    std::vector<double> cost;
+    for (size_t c = 0; c < n; ++c) {
+        const int* m = c < u.ncand ? &u.mbox[4 * c] : none;
+        int* ys = &b.ys[c * nb];
+        if (c > 0 && c < u.ncand && std::equal(m, m + 4, m - 4)) std::copy(ys - nb, ys, ys);
+        else if (!cut_slabs<Real>(pc, p, m, cost, ys)) return;
+        int tall = 0;
+        for (int k = 0; k < p.blocks; ++k) tall = std::max(tall, ys[k + 1] - ys[k]);
+        b.warps = std::max(b.warps, (tall + kRows - 1) / kRows);
+        for (int k = 0; k < p.blocks; ++k)
+            b.smem = std::max(b.smem, resident_layout<Real>(pc.nx, pc.ny, pc.nc, pc.nmat, ref, p.passes, ys[k], ys[k + 1],
+                                                            tall, m[0], m[1], m[2], m[3], d)
+                                          .total);
+    }
+    b.smem = (b.smem + 4095) / 4096 * 4096;   // one captured launch serves batches of about the same boxes
+    b.fits = b.smem <= kSmemPerBlock;
+}
+
+template <typename Real>
+void make_resident(const ProblemClass& pc, const SolveLayout& lay, const ResidentPlan& p, const ResidentBatch& b,
+                   const Unpacked& u, SolveDesc<Real>* descs, int nsolves) {
+    for (int sv = 0; sv < nsolves; ++sv) {
+        SolveDesc<Real>& D = descs[sv];
+        Real* const f = D.ez[0];
+        const size_t fe = lay.field_elems, cand = (size_t)(sv / pc.n_exc);
+        D.resident = 1;
+        D.ez[0] = D.ez[1] = f;
+        D.hx[0] = D.hx[1] = f + fe;
+        D.hy[0] = D.hy[1] = f + 2 * fe;
+        D.jp[0] = D.jp[1] = f + 3 * fe;
+        D.psi[1] = D.psi[0];
+        D.stage = f + 4 * fe;
+        D.mx0 = 1; D.mx1 = 0; D.my0 = 1; D.my1 = 0;
+        if (cand < u.ncand) {
+            const int* m = &u.mbox[4 * cand];
+            D.mx0 = m[0]; D.mx1 = m[1]; D.my0 = m[2]; D.my1 = m[3];
+        }
+        const int* ys = &b.ys[std::min(cand, u.ncand + pc.extra - 1) * (p.blocks + 1)];
+        std::copy(ys, ys + p.blocks + 1, D.ys);
+    }
+}
+
+static cudaLaunchConfig_t cluster_config(const ResidentPlan& p, const ResidentBatch& b, int clusters, cudaStream_t st,
+                                         cudaLaunchAttribute* attr) {
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(clusters * p.blocks);
+    c.blockDim = dim3(32 * b.warps);
+    c.dynamicSmemBytes = b.smem;
+    c.stream = st;
+    attr->id = cudaLaunchAttributeClusterDimension;
+    attr->val.clusterDim.x = p.blocks;
+    attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+    c.attrs = attr;
+    c.numAttrs = 1;
+    return c;
+}
+
+template <typename Real>
+int resident_clusters(const ResidentPlan& p, const ResidentBatch& b, int mode, int* clusters) {
+    ResidentFn<Real> fn = resident_kernel_for<Real>(p.passes, mode);
+    if (!fn) return fail(TOMO_EINVAL, "no resident kernel for this grid");
+    CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemPerBlock));
+    CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    cudaLaunchAttribute attr;
+    cudaLaunchConfig_t c = cluster_config(p, b, 1, nullptr, &attr);
+    CUDA_TRY(cudaOccupancyMaxActiveClusters(clusters, fn, &c));
+    if (*clusters < 1) return fail(TOMO_ECUDA, "a cluster of " + std::to_string(p.blocks) + " blocks does not fit the GPU");
+    return TOMO_OK;
+}
+
+template <typename Real>
+int launch_resident(const ResidentPlan& p, const ResidentBatch& b, int mode, int clusters, const SolveDesc<Real>* descs,
+                    int nsolves, int nsteps, int* error, cudaStream_t st) {
+    ResidentFn<Real> fn = resident_kernel_for<Real>(p.passes, mode);
+    cudaLaunchAttribute attr;
+    cudaLaunchConfig_t c = cluster_config(p, b, std::min(clusters, nsolves), st, &attr);
+    CUDA_TRY(cudaLaunchKernelEx(&c, fn, descs, nsolves, nsteps, error));
+    return TOMO_OK;
+}
+
+#define TOMO_RESIDENT(Real)                                                                                            \
+    template bool resident_plan<Real>(const ProblemClass&, const SolveLayout&, int, ResidentPlan&);                    \
+    template void resident_batch<Real>(const ProblemClass&, const ResidentPlan&, const Unpacked&, ResidentBatch&);     \
+    template void make_resident<Real>(const ProblemClass&, const SolveLayout&, const ResidentPlan&,                    \
+                                      const ResidentBatch&, const Unpacked&, SolveDesc<Real>*, int);                   \
+    template int resident_clusters<Real>(const ResidentPlan&, const ResidentBatch&, int, int*);                        \
+    template int launch_resident<Real>(const ResidentPlan&, const ResidentBatch&, int, int, const SolveDesc<Real>*,    \
+                                       int, int, int*, cudaStream_t);
+TOMO_RESIDENT(float)
+TOMO_RESIDENT(double)
+#undef TOMO_RESIDENT
+
+}  // namespace tomo

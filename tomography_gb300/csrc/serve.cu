@@ -73,7 +73,7 @@ struct ServeStateT {
     size_t smem = 0;
     int hi_slot = 0;   // one past the highest slot ever used
     Blocking blk{0, 0, 0};   // blocking of the serving loop, fixed at the first serving step
-    int cmax = 0;             // largest NTFF contour among the running requests
+    int cmax = 0, fmax = 1;   // largest NTFF contour and most frequencies among the running requests
 
     int find_range(int n) {
         int run = 0;
@@ -319,7 +319,8 @@ int EngineT<Real>::serve_step(int* n_active) {
     int rc;
     ServeStateT<Real>* st = serve_state(serve_, &rc);
     if (!st) return rc;
-    if (st->blk.T == 0) st->blk = blk_;   // the blocking stays fixed while requests are in flight
+    if (st->blk.T == 0)   // the blocking stays fixed while requests are in flight
+        st->blk = blk_.blocks > 0 ? tune_candidates<Real>(advance_mode(cd_.pc.spec), 0, 0, 0).front() : blk_;
     // 1. admit queued requests in arrival order
     while (!st->queue.empty()) {
         auto it = st->reqs.find(st->queue.front());
@@ -353,6 +354,7 @@ int EngineT<Real>::serve_step(int* n_active) {
         }
         const int nseg = choose_segments(strips, nymax, st->blk.T, 24L * num_sms_);
         st->cmax = 0;
+        st->fmax = 1;
         for (auto& kv : st->reqs) {
             const ServeRequest<Real>& r = *kv.second;
             if (r.state != kRunning) continue;
@@ -362,6 +364,7 @@ int EngineT<Real>::serve_step(int* n_active) {
                          st->blk.cols, nseg);
             TOMO_TRY(validate_items(items, n0, pc.nx, pc.ny, pc.nc, item_face_distance(pc), st->blk.T, st->blk.cols));
             st->cmax = std::max(st->cmax, dft_contour(pc));
+            st->fmax = std::max(st->fmax, pc.nfreq);
         }
         st->nitems = (int)items.size();
         if (!items.empty()) {
@@ -392,7 +395,7 @@ int EngineT<Real>::serve_step(int* n_active) {
         for (int l = 0; l < nl; ++l)
             launch_advance<Real>(st->blk, advance_mode(cd_.pc.spec), st->blocks, st->smem,
                                  st->descs.template as<SolveDesc<Real>>(), st->items.template as<WorkItem>(),
-                                 st->nitems, st->hi_slot, d_counter_.as<int>(), st->cmax, stream_);
+                                 st->nitems, st->hi_slot, d_counter_.as<int>(), st->cmax, st->fmax, stream_);
         CUDA_TRY(cudaGetLastError());
         for (auto& kv : st->reqs) {
             ServeRequest<Real>& r = *kv.second;

@@ -24,6 +24,7 @@ constexpr int kMatPadLeft = 32;  // bytes of padding left of x = 0 in every mate
 constexpr int kMaxMat = 128;     // material indices per solve (7 bits)
 constexpr int kMatCoef = 8;      // coefficient columns, see MatCol
 constexpr int kMaxRx = 64;
+constexpr int kMaxSlabs = 16;    // most blocks of a cluster that share one solve
 constexpr int kMaxCpml = 32;     // CPML cells per side (the profile lives in shared memory)
 
 enum SolveFlags : int {
@@ -53,6 +54,9 @@ struct SolveDesc {
     int active;                  // 0: skip this solve
     int nmat;                    // materials in use: indices 0 .. nmat-1 of mtab
     int stage_group;             // launches that fill the contour staging buffer before one DFT pass
+    int resident;                // 1: advanced by the resident kernel (fields stay in copy 0)
+    int mx0, mx1, my0, my1;      // box of every cell that is not background (empty: mx0 > mx1)
+    int ys[kMaxSlabs + 1];       // resident kernel: first row of each block's slab, then ny
     Real chez;                   // dt/(mu0 dx)
     Real Kp;                     // Debye recursion coefficient
     Real dx;
