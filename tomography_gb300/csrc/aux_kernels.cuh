@@ -4,6 +4,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include "packed.cuh"
 #include "solve_desc.h"
 
 namespace tomo {
@@ -159,52 +160,204 @@ __global__ void farfield_kernel(const Real* __restrict__ acc, size_t acc_stride,
 }
 
 // ---------------------------------------------------------------------------
-// Trace misfit partials per solve: num = sum (s - t)^2, den = sum t^2 (FP64).
-template <typename Real>
-__global__ void trace_partials_kernel(const Real* __restrict__ traces, size_t tr_stride, const float* __restrict__ target,
-                                      int n_per_solve, int n_tx, int tx_offset_mod, double* __restrict__ partials,
-                                      int* __restrict__ nonfinite) {
-    const int s = blockIdx.x;
-    const int tx = s % n_tx;
-    const Real* tr = traces + (size_t)s * tr_stride;
-    const float* tg = target + (size_t)tx * n_per_solve;
-    double num = 0, den = 0;
-    int bad = 0;
-    for (int i = threadIdx.x; i < n_per_solve; i += blockDim.x) {
-        const double sv = (double)tr[i], tv = (double)tg[i];
-        if (!isfinite(sv)) bad = 1;
-        num += (sv - tv) * (sv - tv);
-        den += tv * tv;
+// Trace misfit: num = sum (s - t)^2 per solve and den = sum t^2 per transmitter.
+//
+// The samples of a solve are cut into chunks of kMisfitChunk, summed one by one
+// and added in order, whether one block takes all chunks of a solve or every
+// chunk has a block of its own: the result does not depend on the batch.
+//
+// FP64 sums were bound by the FP64 units (two lanes a clock and SM, five
+// operations a sample: 596 us for 49 M samples, 5% of HBM; now 87 us, bound by
+// some 26 FP32 operations a sample).  FP32 traces are
+// summed in FP32 without their rounding errors instead: the difference, its
+// square and every addition are split into a value and its exact error (Knuth's
+// two-sum, an fma for the product), the errors are added up beside the values,
+// and a chunk's sums join in FP64.  A term keeps about 47 bits, whose rounding
+// averages out below an FP64 sum's own.  A chunk whose sum is outside [2^-70, 2^100] -- where products
+// would lose bits to underflow or overflow -- or not finite is done in FP64.
+constexpr int kMisfitChunk = 8192;
+inline int misfit_chunks(size_t n_per_solve) { return (int)((n_per_solve + kMisfitChunk - 1) / kMisfitChunk); }
+
+// A sum, its error and that error's error, two columns of each.
+struct SplitSum {
+    Two<float> sum{0.0f, 0.0f}, err{0.0f, 0.0f}, rest{0.0f, 0.0f};
+    // adds -m + e, with m the negative of a rounded product and e its error
+    __device__ __forceinline__ void take(Two<float> m, Two<float> e) {
+        const Two<float> x = sub2(sum, m), bv = sub2(sum, x), av = add2(x, bv);
+        const Two<float> y = add2(sub2(sum, av), sub2(bv, m));
+        sum = x;
+        const Two<float> f = add2(y, e), z = add2(err, f), fv = sub2(z, err), ev = sub2(z, fv);
+        rest = add2(rest, add2(sub2(err, ev), sub2(f, fv)));
+        err = z;
     }
-    __shared__ double sn[32], sd[32];
-    for (int o = 16; o > 0; o >>= 1) {
-        num += __shfl_xor_sync(0xffffffffu, num, o);
-        den += __shfl_xor_sync(0xffffffffu, den, o);
+    // adds (a - b)^2
+    __device__ __forceinline__ void square_difference(Two<float> a, Two<float> b) {
+        const Two<float> d = sub2(a, b), bv = sub2(a, d), av = add2(d, bv);
+        const Two<float> lo = add2(sub2(a, av), sub2(bv, b));
+        const Two<float> m{__fmul_rn(-d.x, d.x), __fmul_rn(-d.y, d.y)};
+        take(m, fma2(add2(d, d), lo, fma2(lo, lo, fma2(d, d, m))));
     }
-    bad = __any_sync(0xffffffffu, bad);
+    __device__ __forceinline__ void square(Two<float> a) {
+        const Two<float> m{__fmul_rn(-a.x, a.x), __fmul_rn(-a.y, a.y)};
+        take(m, fma2(a, a, m));
+    }
+    // The block's sum in FP64 (thread 0): lanes, then the eight warps, in three parts.
+    // (In two, the few last additions of the errors would round at 2^-49 of the sum.)
+    __device__ __forceinline__ double block_total(float (*part)[3]) const {
+        float s = sum.x, e = err.x, r = rest.x;
+        auto two_sum = [](float& a, float b) {   // a += b; returns the rounding error
+            const float x = __fadd_rn(a, b), bv = __fsub_rn(x, a), av = __fsub_rn(x, bv);
+            const float y = __fadd_rn(__fsub_rn(a, av), __fsub_rn(b, bv));
+            a = x;
+            return y;
+        };
+        auto add = [&](float b, float f, float g) {
+            const float y = two_sum(s, b);
+            r = __fadd_rn(r, __fadd_rn(g, two_sum(e, f)));
+            r = __fadd_rn(r, two_sum(e, y));
+        };
+        auto across = [&](int o) {
+            const float b = __shfl_xor_sync(0xffffffffu, s, o), f = __shfl_xor_sync(0xffffffffu, e, o),
+                        g = __shfl_xor_sync(0xffffffffu, r, o);
+            add(b, f, g);
+        };
+        add(sum.y, err.y, rest.y);
+        for (int o = 16; o > 0; o >>= 1) across(o);
+        __syncthreads();
+        if ((threadIdx.x & 31) == 0) {
+            float* q = part[threadIdx.x >> 5];
+            q[0] = s; q[1] = e; q[2] = r;
+        }
+        __syncthreads();
+        if (threadIdx.x < 32) {
+            const float* q = part[threadIdx.x & 7];
+            s = q[0]; e = q[1]; r = q[2];
+            for (int o = 4; o > 0; o >>= 1) across(o);
+        }
+        return (double)s + ((double)e + (double)r);
+    }
+};
+
+// Sum over the block of one value per warp, in warp order (thread 0).
+__device__ __forceinline__ double misfit_join(double v, double* part) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    if (lane == 0) { sn[w] = num; sd[w] = den; }
-    if (bad && lane == 0) atomicOr(nonfinite, 1);
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double a = 0, b = 0;
-        for (int i = 0; i < (int)(blockDim.x >> 5); ++i) { a += sn[i]; b += sd[i]; }
-        partials[2 * s] = a;
-        partials[2 * s + 1] = b;
-    }
-    (void)tx_offset_mod;
+    if (lane == 0) part[w] = v;
+    __syncthreads();
+    double a = 0;
+    if (threadIdx.x == 0)
+        for (int i = 0; i < (int)(blockDim.x >> 5); ++i) a += part[i];
+    return a;
 }
 
-// fitness[c] = -sum_tx num / sum_tx den, summed in transmitter order.
-static __global__ void trace_fitness_kernel(const double* __restrict__ partials, int n_tx, int ncand, double* fitness) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+// One chunk in FP64: the general form.
+template <typename Real>
+__device__ inline void misfit_chunk_fp64(const Real* tr, const float* tg, int n, double* part, double* num, double* den,
+                                         int* nonfinite) {
+    double a = 0, b = 0;
+    int bad = 0;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        const double sv = (double)tr[i], tv = (double)tg[i];
+        if (!isfinite(sv)) bad = 1;
+        a += (sv - tv) * (sv - tv);
+        if (den) b += tv * tv;
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        a += __shfl_xor_sync(0xffffffffu, a, o);
+        b += __shfl_xor_sync(0xffffffffu, b, o);
+    }
+    bad = __any_sync(0xffffffffu, bad);
+    if (bad && (threadIdx.x & 31) == 0) atomicOr(nonfinite, 1);
+    *num = misfit_join(a, part);
+    if (den) *den = misfit_join(b, part);
+}
+
+// One chunk of FP32 traces with split sums; false when its sums ask for FP64.
+__device__ inline bool misfit_chunk_split(const float* tr, const float* tg, int n, bool aligned, double* part,
+                                          double* num, double* den) {
+    SplitSum d, t;
+    // the same samples to the same threads whatever the alignment
+    auto four = [&](const float* p, int i) {
+        return aligned ? __ldg(reinterpret_cast<const float4*>(p) + i)
+                       : make_float4(__ldg(p + 4 * i), __ldg(p + 4 * i + 1), __ldg(p + 4 * i + 2), __ldg(p + 4 * i + 3));
+    };
+    const int quads = n / 4;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < quads; i += blockDim.x) {
+        const float4 a = four(tr, i), b = four(tg, i);
+        d.square_difference({a.x, a.y}, {b.x, b.y});
+        d.square_difference({a.z, a.w}, {b.z, b.w});
+        if (den) {
+            t.square({b.x, b.y});
+            t.square({b.z, b.w});
+        }
+    }
+    for (int i = 4 * quads + threadIdx.x; i < n; i += blockDim.x) {
+        d.square_difference({tr[i], 0.0f}, {tg[i], 0.0f});
+        if (den) t.square({tg[i], 0.0f});
+    }
+    float(*const parts)[3] = reinterpret_cast<float(*)[3]>(part);
+    *num = d.block_total(parts);
+    if (den) *den = t.block_total(parts);
+    auto safe = [](double v) { return v >= 0x1p-70 && v <= 0x1p100; };
+    return __syncthreads_and(threadIdx.x != 0 || (safe(*num) && (!den || safe(*den))));
+}
+
+// num [nsolves][parts] and den [n_tx][parts]: gridDim.y = parts blocks per solve
+// (parts = the solve's chunks), or one block that adds them all up (parts = 1).
+// The target's own sum is taken once, by the first candidate's solves.
+template <typename Real>
+__global__ void __launch_bounds__(256)
+    trace_partials_kernel(const Real* __restrict__ traces, size_t tr_stride, const float* __restrict__ target,
+                          int n_per_solve, int n_tx, double* __restrict__ num, double* __restrict__ den,
+                          int* __restrict__ nonfinite) {
+    __shared__ double part[12];   // eight warps' FP64 sums, or three floats each
+    const int s = blockIdx.x, tx = s % n_tx, parts = gridDim.y, chunks = (n_per_solve + kMisfitChunk - 1) / kMisfitChunk;
+    const bool with_den = s < n_tx;
+    double a = 0, b = 0;
+    for (int c = blockIdx.y; c < chunks; c += parts) {
+        const size_t at = (size_t)c * kMisfitChunk;
+        const int n = min(kMisfitChunk, n_per_solve - (int)at);
+        const Real* tr = traces + (size_t)s * tr_stride + at;
+        const float* tg = target + (size_t)tx * n_per_solve + at;
+        double cn = 0, cd = 0;
+        bool done = false;
+        if constexpr (sizeof(Real) == 4) {
+            const bool aligned = (((size_t)tr | (size_t)tg) & 15) == 0;
+            done = misfit_chunk_split(tr, tg, n, aligned, part, &cn, with_den ? &cd : nullptr);
+        }
+        if (!done) misfit_chunk_fp64<Real>(tr, tg, n, part, &cn, with_den ? &cd : nullptr, nonfinite);
+        a += cn;
+        b += cd;
+    }
+    if (threadIdx.x == 0) {
+        num[(size_t)s * parts + blockIdx.y] = a;
+        if (with_den) den[(size_t)tx * parts + blockIdx.y] = b;
+    }
+}
+
+// fitness[c] = -sum_tx num / sum_tx den: a warp per candidate, a transmitter's
+// chunks in order, then the lanes' transmitters.
+static __global__ void trace_fitness_kernel(const double* __restrict__ num, const double* __restrict__ den, int parts,
+                                            int n_tx, int ncand, double* fitness) {
+    const int c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (c >= ncand) return;
     double a = 0, b = 0;
-    for (int t = 0; t < n_tx; ++t) {
-        a += partials[2 * (c * n_tx + t)];
-        b += partials[2 * (c * n_tx + t) + 1];
+    for (int t = lane; t < n_tx; t += 32) {
+        double p = 0, q = 0;
+#pragma unroll 8
+        for (int k = 0; k < parts; ++k) {
+            p += num[(size_t)(c * n_tx + t) * parts + k];
+            q += den[(size_t)t * parts + k];
+        }
+        a += p;
+        b += q;
     }
-    fitness[c] = b > 0 ? -a / b : -a;
+    for (int o = 16; o > 0; o >>= 1) {
+        a += __shfl_xor_sync(0xffffffffu, a, o);
+        b += __shfl_xor_sync(0xffffffffu, b, o);
+    }
+    if (lane == 0) fitness[c] = b > 0 ? -a / b : -a;
 }
 
 // Far-field misfit (FDTD_GPU.cu:1004-1022 absolute; FDTD_CPU.cxx:841-845 relative).

@@ -352,8 +352,10 @@ int post_range(const ClassData<Real>& cd, size_t ncand, const SolveDesc<Real>& f
     if (want_fit) {
         if (s.mode == TOMO_MODE_BREAST) {
             trace_partials_kernel<Real><<<nsolves, 256, 0, st>>>(first.traces, stride, cd.target.template as<float>(),
-                                                                 pc.nrx * pc.S, pc.n_exc, 0, d_partials, d_flag);
-            trace_fitness_kernel<<<(int)((ncand + 127) / 128), 128, 0, st>>>(d_partials, pc.n_exc, (int)ncand, d_fit);
+                                                                 pc.nrx * pc.S, pc.n_exc, d_partials,
+                                                                 d_partials + nsolves, d_flag);
+            trace_fitness_kernel<<<(int)((ncand + 3) / 4), 128, 0, st>>>(d_partials, d_partials + nsolves, 1, pc.n_exc,
+                                                                          (int)ncand, d_fit);
             *kernels += 2;
         } else {
             const int nper = pc.n_exc * pc.nfreq * pc.nang;

@@ -30,6 +30,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include "fdtd_advance.cuh"
+#include "packed.cuh"
 #include "solve_desc.h"
 
 namespace tomo {
@@ -40,65 +41,6 @@ constexpr int kRows = 4;             // rows per warp
 // fill the registers, of which 8 warps leave 255 a thread and 12 leave 168.
 constexpr int resident_warps(int passes) { return passes == 1 ? 12 : 8; }
 constexpr int kResidentWarps = 12;
-
-// Two values of one operation: a packed f32x2 instruction in FP32 (the same
-// rounding per half as the scalar form), two scalar ones in FP64.
-template <typename Real>
-struct alignas(2 * sizeof(Real)) Two {
-    Real x, y;
-};
-__device__ __forceinline__ unsigned long long two_bits(Two<float> a) {
-    unsigned long long r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a.x), "f"(a.y));
-    return r;
-}
-__device__ __forceinline__ Two<float> two_of(unsigned long long v) {
-    Two<float> r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
-__device__ __forceinline__ Two<float> add2(Two<float> a, Two<float> b) {
-    unsigned long long r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(two_bits(a)), "l"(two_bits(b)));
-    return two_of(r);
-}
-__device__ __forceinline__ Two<float> sub2(Two<float> a, Two<float> b) {
-    unsigned long long r;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(two_bits(a)), "l"(two_bits(b)));
-    return two_of(r);
-}
-__device__ __forceinline__ Two<float> fma2(Two<float> a, Two<float> b, Two<float> c) {
-    unsigned long long r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(two_bits(a)), "l"(two_bits(b)), "l"(two_bits(c)));
-    return two_of(r);
-}
-// A packed product must not feed a packed sum or difference: the compiler may
-// fuse the two.  Such products are written as scalar ones (times2).
-__device__ __forceinline__ Two<float> mul2(Two<float> a, Two<float> b) {
-    unsigned long long r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(two_bits(a)), "l"(two_bits(b)));
-    return two_of(r);
-}
-__device__ __forceinline__ Two<double> add2(Two<double> a, Two<double> b) {
-    return {__dadd_rn(a.x, b.x), __dadd_rn(a.y, b.y)};
-}
-__device__ __forceinline__ Two<double> sub2(Two<double> a, Two<double> b) {
-    return {__dsub_rn(a.x, b.x), __dsub_rn(a.y, b.y)};
-}
-__device__ __forceinline__ Two<double> mul2(Two<double> a, Two<double> b) {
-    return {__dmul_rn(a.x, b.x), __dmul_rn(a.y, b.y)};
-}
-__device__ __forceinline__ Two<double> fma2(Two<double> a, Two<double> b, Two<double> c) {
-    return {__fma_rn(a.x, b.x, c.x), __fma_rn(a.y, b.y, c.y)};
-}
-template <typename Real>
-__device__ __forceinline__ Two<Real> times2(Two<Real> a, Two<Real> b) {
-    return {Op<Real>::mul(a.x, b.x), Op<Real>::mul(a.y, b.y)};
-}
-template <typename Real>
-__device__ __forceinline__ Two<Real> dup2(Real v) {
-    return {v, v};
-}
 
 // 16 bytes of a row: the columns of one lane in a pass.
 template <typename Real>

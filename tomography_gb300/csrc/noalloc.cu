@@ -89,9 +89,16 @@ extern "C" int tomo_trace_misfit_static(const float* traces, const float* target
         const int nsolves = (int)(n_cand * n_tx);
         e = cudaMemsetAsync(flag, 0, sizeof(int) * 4, st);   // the flag must start at zero every call
         if (e != cudaSuccess) return fail(TOMO_ECUDA, std::string("cudaMemsetAsync: ") + cudaGetErrorString(e));
-        tomo::trace_partials_kernel<float><<<nsolves, 256, 0, st>>>(traces, n_per_solve, target, (int)n_per_solve,
-                                                                    (int)n_tx, 0, partials, flag);
-        tomo::trace_fitness_kernel<<<(int)((n_cand + 127) / 128), 128, 0, st>>>(partials, (int)n_tx, (int)n_cand, fitness);
+        // a block for every chunk of a solve where the scratch holds their sums (the first
+        // half the solves', the second the transmitters'): a few solves then fill the GPU
+        const size_t chunks = (size_t)tomo::misfit_chunks(n_per_solve);
+        const int parts = chunks * n_cand * n_tx <= tomo::kNoAllocMaxSolves ? (int)chunks : 1;
+        double* const den = partials + tomo::kNoAllocMaxSolves;
+        tomo::trace_partials_kernel<float><<<dim3(nsolves, parts), 256, 0, st>>>(traces, n_per_solve, target,
+                                                                                 (int)n_per_solve, (int)n_tx, partials,
+                                                                                 den, flag);
+        tomo::trace_fitness_kernel<<<(int)((n_cand + 3) / 4), 128, 0, st>>>(partials, den, parts, (int)n_tx, (int)n_cand,
+                                                                             fitness);
         e = cudaGetLastError();
         if (e != cudaSuccess) return fail(TOMO_ECUDA, std::string("misfit launch: ") + cudaGetErrorString(e));
         return TOMO_OK;
