@@ -74,14 +74,15 @@ __global__ void material_table_kernel(const double* __restrict__ mp, Real* __res
     out[kCs] = (Real)((-2 * dt) / den);
 }
 
-// Progress every active solve by T steps after an advance launch.
+// Progress every active solve of one kind (wavefront or resident) by T steps after
+// an advance launch; counter may be null.
 template <typename Real>
-__global__ void bump_kernel(SolveDesc<Real>* descs, int nsolves, int T, int* counter) {
+__global__ void bump_kernel(SolveDesc<Real>* descs, int nsolves, int T, int* counter, int resident) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s == 0) *counter = 0;   // work counter of the next advance launch
+    if (s == 0 && counter) *counter = 0;   // work counter of the next advance launch
     if (s >= nsolves) return;
     SolveDesc<Real>& D = descs[s];
-    if (D.active && D.step < D.steps_total) {
+    if (D.active && D.resident == resident && D.step < D.steps_total) {
         D.step += T;
         if (!D.resident) D.parity ^= 1;   // the resident kernel keeps its state in one copy
     }

@@ -790,9 +790,9 @@ int EngineT<Real>::build_graph(int nlaunch) {
                                    d_counter_.as<int>() + 1, stream_);
         if (dft_contour(cd_.pc) > 0)
             launch_dft<Real>(d_descs_.as<SolveDesc<Real>>(), nsolves_, dft_contour(cd_.pc), cd_.pc.nfreq, T, l * T,
-                             std::min(T, S - l * T), stream_);
+                             std::min(T, S - l * T), 1, stream_);
         bump_kernel<Real><<<(nsolves_ + 127) / 128, 128, 0, stream_>>>(d_descs_.as<SolveDesc<Real>>(), nsolves_, T,
-                                                                       d_counter_.as<int>());
+                                                                       nullptr, 1);
     }
     for (int l = 0; !resident && l < nlaunch; ++l) {
         const bool last_of_group = (l + 1) % group == 0 || l == nlaunch - 1;

@@ -423,6 +423,7 @@ struct ResidentBatch {
     int warps = 0;             // per block
     size_t smem = 0;           // per block
     std::vector<int> ys;       // [ncand (+ 1)][blocks + 1]: first row of each slab, then ny
+    double cost = 0;           // of the dearest slab
 };
 // false: the class does not fit the resident kernel with that many blocks.
 template <typename Real>
@@ -436,6 +437,11 @@ void resident_batch(const ProblemClass& pc, const ResidentPlan& p, const Unpacke
 template <typename Real>
 void make_resident(const ProblemClass& pc, const SolveLayout& lay, const ResidentPlan& p, const ResidentBatch& b,
                    const Unpacked& u, SolveDesc<Real>* descs, int nsolves);
+// Of the plans that fit, the one whose launch should take least (no measuring:
+// the serving loop admits requests of any size at any time).  -1: none fits.
+template <typename Real>
+int resident_choice(const ProblemClass& pc, const SolveLayout& lay, const Unpacked& u, ResidentPlan& p,
+                    ResidentBatch& b);
 // Clusters of the batch that run at once, and one launch of nsteps steps.
 template <typename Real>
 int resident_clusters(const ResidentPlan& p, const ResidentBatch& b, int mode, int* clusters);
@@ -454,8 +460,9 @@ inline int stage_group_for(int T) { return std::max(1, kStageLevels / std::max(T
 
 template <typename Real>
 void launch_dft(const SolveDesc<Real>* descs, int nsolves, int cmax, int fmax, int T, int n0, int nlev,
-                cudaStream_t st) {
-    dft_accumulate_kernel<Real><<<dim3(nsolves * fmax, (cmax + 127) / 128), 128, 0, st>>>(descs, T, fmax, n0, nlev);
+                int resident, cudaStream_t st) {
+    dft_accumulate_kernel<Real><<<dim3(nsolves * fmax, (cmax + 127) / 128), 128, 0, st>>>(descs, T, fmax, n0, nlev,
+                                                                                              resident);
 }
 
 // One advance launch (T steps of every listed solve), then -- when cmax, the
@@ -471,9 +478,9 @@ int launch_advance(const Blocking& b, int mode, int blocks, size_t smem, const S
     fn<<<blocks, 128, smem, st>>>(descs, items, nitems, counter);
     const bool dft = cmax > 0 && dft_nlev != 0;
     if (dft)
-        launch_dft<Real>(descs, nsolves, cmax, fmax, b.T, dft_n0, dft_nlev, st);
+        launch_dft<Real>(descs, nsolves, cmax, fmax, b.T, dft_n0, dft_nlev, 0, st);
     bump_kernel<Real><<<(nsolves + 127) / 128, 128, 0, st>>>(const_cast<SolveDesc<Real>*>(descs), nsolves, b.T,
-                                                            counter);
+                                                            counter, 0);
     return dft ? 3 : 2;
 }
 

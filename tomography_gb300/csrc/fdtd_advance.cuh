@@ -209,12 +209,12 @@ constexpr int kStageLevels = 8;
 
 template <typename Real>
 __global__ void __launch_bounds__(128) dft_accumulate_kernel(const SolveDesc<Real>* __restrict__ descs, int T,
-                                                             int fmax, int n0_group, int nlev) {
+                                                             int fmax, int n0_group, int nlev, int resident) {
     const SolveDesc<Real>& D = descs[blockIdx.x / fmax];
     const int f = blockIdx.x % fmax;
     const int c = blockIdx.y * blockDim.x + threadIdx.x;
     const int C = D.n_contour, nfreq = D.nfreq;
-    if (!D.active || f >= nfreq || c >= C) return;
+    if (!D.active || D.resident != resident || f >= nfreq || c >= C) return;
     const int n0 = n0_group >= 0 ? n0_group : D.step;
     const int nsteps = min(n0_group >= 0 ? nlev : T, D.steps_total - n0);
     Real* a = D.acc + ((size_t)f * C + c) * 8;

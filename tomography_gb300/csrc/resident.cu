@@ -33,7 +33,8 @@ bool resident_plan(const ProblemClass& pc, const SolveLayout& lay, int blocks, R
 // Cuts rows 1 .. ny-1 into slabs of about equal cost: the least cost of the
 // dearest slab, by bisection over a greedy cut.  box: the candidate's materials.
 template <typename Real>
-static bool cut_slabs(const ProblemClass& pc, const ResidentPlan& p, const int* box, std::vector<double>& cost, int* ys) {
+static bool cut_slabs(const ProblemClass& pc, const ResidentPlan& p, const int* box, std::vector<double>& cost, int* ys,
+                      double& dearest) {
     const int most = kRows * resident_warps(p.passes), width = 32 * Quad<Real>::N;
     // cost of a row, from the passes' measured times: a plain pass 0.14, one with
     // materials or y-CPML 0.42, the rest of a row 0.6
@@ -77,6 +78,7 @@ static bool cut_slabs(const ProblemClass& pc, const ResidentPlan& p, const int* 
         else lo = mid;
     }
     if (!cut(hi)) return false;
+    dearest = std::max(dearest, hi);
     for (int b = 0; b < p.blocks; ++b)
         if (ys[b + 1] - ys[b] < 2) return false;
     return true;
@@ -90,13 +92,14 @@ void resident_batch(const ProblemClass& pc, const ResidentPlan& p, const Unpacke
     b.fits = false;
     b.warps = 0;
     b.smem = 0;
+    b.cost = 0;
     b.ys.resize(n * nb);
     std::vector<double> cost;
     for (size_t c = 0; c < n; ++c) {
         const int* m = c < u.ncand ? &u.mbox[4 * c] : none;
         int* ys = &b.ys[c * nb];
         if (c > 0 && c < u.ncand && std::equal(m, m + 4, m - 4)) std::copy(ys - nb, ys, ys);
-        else if (!cut_slabs<Real>(pc, p, m, cost, ys)) return;
+        else if (!cut_slabs<Real>(pc, p, m, cost, ys, b.cost)) return;
         int tall = 0;
         for (int k = 0; k < p.blocks; ++k) tall = std::max(tall, ys[k + 1] - ys[k]);
         b.warps = std::max(b.warps, (tall + kRows - 1) / kRows);
@@ -162,6 +165,31 @@ int resident_clusters(const ResidentPlan& p, const ResidentBatch& b, int mode, i
 }
 
 template <typename Real>
+int resident_choice(const ProblemClass& pc, const SolveLayout& lay, const Unpacked& u, ResidentPlan& p,
+                    ResidentBatch& b) {
+    int best = -1;
+    double least = 0;
+    for (int blocks : {16, 8, 4}) {
+        ResidentPlan q;
+        if (!resident_plan<Real>(pc, lay, blocks, q)) continue;
+        ResidentBatch c;
+        resident_batch<Real>(pc, q, u, c);
+        int clusters = 0;
+        if (!c.fits || resident_clusters<Real>(q, c, advance_mode(pc.spec), &clusters)) continue;
+        // rounds of clusters, each about 1 us a step and 0.06 us per unit of the dearest slab
+        const int nsolves = (int)u.ncand * pc.n_exc;
+        const double t = ((nsolves + clusters - 1) / clusters) * (1.0 + 0.06 * c.cost);
+        if (best < 0 || t < least) {
+            best = blocks;
+            least = t;
+            p = q;
+            b = c;
+        }
+    }
+    return best;
+}
+
+template <typename Real>
 int launch_resident(const ResidentPlan& p, const ResidentBatch& b, int mode, int clusters, const SolveDesc<Real>* descs,
                     int nsolves, int nsteps, int* error, cudaStream_t st) {
     ResidentFn<Real> fn = resident_kernel_for<Real>(p.passes, mode);
@@ -176,6 +204,8 @@ int launch_resident(const ResidentPlan& p, const ResidentBatch& b, int mode, int
     template void resident_batch<Real>(const ProblemClass&, const ResidentPlan&, const Unpacked&, ResidentBatch&);     \
     template void make_resident<Real>(const ProblemClass&, const SolveLayout&, const ResidentPlan&,                    \
                                       const ResidentBatch&, const Unpacked&, SolveDesc<Real>*, int);                   \
+    template int resident_choice<Real>(const ProblemClass&, const SolveLayout&, const Unpacked&, ResidentPlan&,        \
+                                       ResidentBatch&);                                                                \
     template int resident_clusters<Real>(const ResidentPlan&, const ResidentBatch&, int, int*);                        \
     template int launch_resident<Real>(const ResidentPlan&, const ResidentBatch&, int, int, const SolveDesc<Real>*,    \
                                        int, int, int*, cudaStream_t);

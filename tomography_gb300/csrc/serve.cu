@@ -7,9 +7,10 @@
 //     n_exc solves; a request may carry its own grid spec);
 //   * tomo_serve_step admits queued requests in FIFO order while their memory
 //     fits the HBM budget and descriptor slots are free, then advances EVERY
-//     admitted solve by up to four launches of the descriptor-driven advance
-//     kernel (solves of different requests, grid sizes and progress share
-//     the launches), and retires requests whose solves reached their last step
+//     admitted solve -- a request that fits the resident kernel by one launch
+//     of it, the others by up to four launches of the descriptor-driven
+//     wavefront kernel (solves of different requests, grid sizes and progress
+//     share the launches) -- and retires requests whose solves reached their last step
 //     (far field + misfit on the device, fitness to the host);
 //   * tomo_poll returns a finished request's fitness.
 // Each solve's arithmetic depends only on its own descriptor, so a result is
@@ -43,6 +44,10 @@ struct ServeRequest {
     int steps_done = 0;
     int status = TOMO_OK;
     Unpacked up;
+    bool resident = false;    // advanced by the resident kernel, else by the wavefront kernel
+    ResidentPlan plan;
+    ResidentBatch batch;
+    int clusters = 0;
     void* mem = nullptr;      // stream-ordered allocation holding everything below
     size_t bytes = 0;
     Real* state_base = nullptr;
@@ -227,7 +232,7 @@ int EngineT<Real>::request_bytes(const tomo_spec* spec, size_t ncand, uint64_t* 
 
 template <typename Real>
 static int admit(EngineT<Real>* eng, ServeStateT<Real>* st, ServeRequest<Real>& r, cudaStream_t stream,
-                 uint64_t budget, bool* admitted) {
+                 uint64_t budget, bool resident, bool* admitted) {
     *admitted = false;
     const ClassData<Real>& cd = *r.cd;
     const RequestLayout lay = request_layout(cd, r.ncand, r.up.upload.size());
@@ -267,6 +272,11 @@ static int admit(EngineT<Real>* eng, ServeStateT<Real>* st, ServeRequest<Real>& 
         CUDA_TRY(cudaMemsetAsync(r.state_base, 0, b_state, stream));
         CUDA_TRY(cudaMemsetAsync(r.flag, 0, sizeof(int), stream));
         fill_descs<Real>(cd, r.up, r.state_base, r.mats, r.tabs, &st->hdescs[first]);
+        r.resident = resident && resident_choice<Real>(cd.pc, cd.lay, r.up, r.plan, r.batch) > 0;
+        if (r.resident) {
+            TOMO_TRY(resident_clusters<Real>(r.plan, r.batch, advance_mode(cd.pc.spec), &r.clusters));
+            make_resident<Real>(cd.pc, cd.lay, r.plan, r.batch, r.up, &st->hdescs[first], r.nsolves);
+        }
         CUDA_TRY(cudaMemcpyAsync(st->descs.template as<SolveDesc<Real>>() + first, &st->hdescs[first],
                                  sizeof(SolveDesc<Real>) * r.nsolves, cudaMemcpyHostToDevice, stream));
         return TOMO_OK;
@@ -329,7 +339,7 @@ int EngineT<Real>::serve_step(int* n_active) {
             continue;
         }
         bool admitted = false;
-        rc = admit(this, st, *it->second, stream_, budget_, &admitted);
+        rc = admit(this, st, *it->second, stream_, budget_, auto_T_ && auto_cols_ && auto_minb_, &admitted);
         if (rc) {
             it->second->state = kFailed;
             it->second->status = rc;
@@ -346,7 +356,7 @@ int EngineT<Real>::serve_step(int* n_active) {
         int nymax = 0;
         for (auto& kv : st->reqs) {
             const ServeRequest<Real>& r = *kv.second;
-            if (r.state != kRunning) continue;
+            if (r.state != kRunning || r.resident) continue;
             const ProblemClass& pc = r.cd->pc;
             strips += (long)r.nsolves * items_per_solve(pc.nx, pc.ny, pc.nc, item_face_distance(pc), st->blk.T,
                                                        st->blk.cols);
@@ -357,7 +367,7 @@ int EngineT<Real>::serve_step(int* n_active) {
         st->fmax = 1;
         for (auto& kv : st->reqs) {
             const ServeRequest<Real>& r = *kv.second;
-            if (r.state != kRunning) continue;
+            if (r.state != kRunning || r.resident) continue;
             const size_t n0 = items.size();
             const ProblemClass& pc = r.cd->pc;
             append_items(items, r.first, r.nsolves, pc.nx, pc.ny, pc.nc, item_face_distance(pc), st->blk.T,
@@ -378,34 +388,50 @@ int EngineT<Real>::serve_step(int* n_active) {
         CUDA_TRY(cudaStreamSynchronize(stream_));
         st->items_dirty = false;
     }
-    // 3. advance launches over everything admitted: as many as the running
-    // request closest to its end still needs, at most kLaunchesPerStep, so
-    // that no request runs past its last step and the host synchronises once
-    // per serving step rather than once per launch
-    constexpr int kLaunchesPerStep = 4;
-    int running = 0;
-    if (st->nitems > 0) {
-        int nl = kLaunchesPerStep;
-        for (auto& kv : st->reqs) {
-            const ServeRequest<Real>& r = *kv.second;
-            if (r.state == kRunning)
-                nl = std::min(nl, (r.cd->pc.S - r.steps_done + st->blk.T - 1) / st->blk.T);
+    // 3. advance everything admitted.  Requests on the resident kernel: one launch
+    // of up to kServeSteps steps each (the kernel ends at a solve's last step).
+    // The others together: as many wavefront launches as the one closest to its
+    // end still needs, at most kLaunchesPerStep, so that no request runs past its
+    // last step.  The host synchronises once per serving step.
+    constexpr int kServeSteps = 128, kLaunchesPerStep = 4;
+    const int mode = advance_mode(cd_.pc.spec);
+    int running = 0, nl = st->nitems > 0 ? kLaunchesPerStep : 0;
+    for (auto& kv : st->reqs) {
+        ServeRequest<Real>& r = *kv.second;
+        if (r.state != kRunning) continue;
+        const ProblemClass& pc = r.cd->pc;
+        if (!r.resident) {
+            nl = std::min(nl, (pc.S - r.steps_done + st->blk.T - 1) / st->blk.T);
+            continue;
         }
-        nl = std::max(nl, 1);
-        for (int l = 0; l < nl; ++l)
-            launch_advance<Real>(st->blk, advance_mode(cd_.pc.spec), st->blocks, st->smem,
-                                 st->descs.template as<SolveDesc<Real>>(), st->items.template as<WorkItem>(),
-                                 st->nitems, st->hi_slot, d_counter_.as<int>(), st->cmax, st->fmax, stream_);
-        CUDA_TRY(cudaGetLastError());
-        for (auto& kv : st->reqs) {
-            ServeRequest<Real>& r = *kv.second;
-            if (r.state != kRunning) continue;
-            r.steps_done += nl * st->blk.T;
-            if (r.steps_done >= r.cd->pc.S) TOMO_TRY(retire(st, r, stream_, true));
-            else ++running;
-        }
+        SolveDesc<Real>* const d = st->descs.template as<SolveDesc<Real>>() + r.first;
+        const int steps = std::min(kServeSteps, r.plan.levels);
+        TOMO_TRY(launch_resident<Real>(r.plan, r.batch, mode, r.clusters, d, r.nsolves, steps, d_counter_.as<int>() + 1,
+                                       stream_));
+        if (dft_contour(pc) > 0)
+            launch_dft<Real>(d, r.nsolves, dft_contour(pc), pc.nfreq, steps, -1, steps, 1, stream_);
+        bump_kernel<Real><<<(r.nsolves + 127) / 128, 128, 0, stream_>>>(d, r.nsolves, steps, nullptr, 1);
+        r.steps_done += steps;
     }
+    for (int l = 0; l < nl; ++l)
+        launch_advance<Real>(st->blk, mode, st->blocks, st->smem, st->descs.template as<SolveDesc<Real>>(),
+                             st->items.template as<WorkItem>(), st->nitems, st->hi_slot, d_counter_.as<int>(), st->cmax,
+                             st->fmax, stream_);
+    CUDA_TRY(cudaGetLastError());
+    for (auto& kv : st->reqs) {
+        ServeRequest<Real>& r = *kv.second;
+        if (r.state != kRunning) continue;
+        if (!r.resident) r.steps_done += nl * st->blk.T;
+        if (r.steps_done >= r.cd->pc.S) TOMO_TRY(retire(st, r, stream_, true));
+        else ++running;
+    }
+    int lost = 0;
+    CUDA_TRY(cudaMemcpyAsync(&lost, d_counter_.as<int>() + 1, sizeof(int), cudaMemcpyDeviceToHost, stream_));
     CUDA_TRY(cudaStreamSynchronize(stream_));
+    if (lost) {
+        CUDA_TRY(cudaMemset(d_counter_.as<int>() + 1, 0, sizeof(int)));
+        return fail(TOMO_ECUDA, "internal error: a halo row of the resident kernel did not arrive");
+    }
     for (auto& kv : st->reqs) {
         ServeRequest<Real>& r = *kv.second;
         if (r.state == kRunning && r.mem == nullptr) {
