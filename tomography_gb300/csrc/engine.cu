@@ -520,7 +520,7 @@ int EngineT<Real>::init(const ProblemClass& pc) {
         return fail(TOMO_EINVAL, "unsupported (steps_per_launch, cols_per_lane) pair for this mode and precision");
     blk_ = c.front();   // until the first batch is tuned
     if (auto_T_ && auto_cols_ && auto_minb_ && !pc.spec.plain)
-        for (int blocks : {16, 8, 4}) {
+        for (int blocks : kClusterSizes) {
             ResidentPlan p;
             if (resident_plan<Real>(cd_.pc, cd_.lay, blocks, p)) plans_.push_back(p);
         }
@@ -548,30 +548,43 @@ int EngineT<Real>::upload_descs(size_t ncand) {
     return TOMO_OK;
 }
 
-// Times every resident plan that fits the batch (the time of a launch of 40
-// steps less that of one of 8: the slabs' loading and storing cancels) and
-// keeps the fastest; blk_ and plan_ are set.
+// Sets blk_ and plan_at_ to the resident plan of a batch, if one fits.  The plan of a
+// batch size is chosen once: of the three with the least estimated time, the fastest
+// measured (a launch of 40 steps less one of 8: the slabs' loading and storing cancels).
+// A batch that the chosen one does not hold takes the one with the least estimate.
 template <typename Real>
-int EngineT<Real>::autotune_resident(size_t ncand) {
+int EngineT<Real>::pick_resident(size_t ncand, bool* fits) {
     constexpr int kShort = 8, kLong = 40;
+    constexpr size_t kTimed = 3;
     const ProblemClass& pc = cd_.pc;
     const int mode = advance_mode(pc.spec), key = (int)ncand * pc.n_exc;
     auto use = [&](size_t i) {
         plan_at_ = i;
         blk_ = Blocking{std::min(plans_[i].levels, pc.S), Quad<Real>::N, 1, plans_[i].blocks};
+        *fits = true;
     };
-    std::vector<size_t> fit;
-    for (size_t i = 0; i < plans_.size(); ++i)
-        if (plan_batch_[i].fits) fit.push_back(i);
     const auto known = tuned_resident_.find(key);
-    if (known != tuned_resident_.end())
-        for (size_t i : fit)
-            if (plans_[i].blocks == known->second.blocks) {
-                use(i);
-                return TOMO_OK;
-            }
-    use(fit.front());
-    if (known != tuned_resident_.end()) return TOMO_OK;   // the tuned one does not fit this batch
+    if (known != tuned_resident_.end()) {
+        resident_batch<Real>(pc, plans_[known->second], up_, plan_batch_[known->second]);
+        if (plan_batch_[known->second].fits) {
+            use(known->second);
+            return TOMO_OK;
+        }
+    }
+    std::vector<std::pair<double, size_t>> rated;
+    for (size_t i = 0; i < plans_.size(); ++i) {
+        int clusters = 0;
+        resident_batch<Real>(pc, plans_[i], up_, plan_batch_[i]);
+        if (!plan_batch_[i].fits) continue;
+        TOMO_TRY(resident_clusters<Real>(plans_[i], plan_batch_[i], mode, &clusters));
+        if (clusters > 0) rated.push_back({resident_estimate(plan_batch_[i], key + (int)pc.extra, clusters), i});
+    }
+    if (rated.empty()) return TOMO_OK;
+    std::sort(rated.begin(), rated.end());
+    use(rated.front().second);
+    if (known != tuned_resident_.end()) return TOMO_OK;
+    std::vector<size_t> fit;
+    for (size_t i = 0; i < std::min(kTimed, rated.size()); ++i) fit.push_back(rated[i].second);
     if (fit.size() > 1 && pc.S >= kShort + kLong) {
         TOMO_TRY(ensure_batch((int)ncand));
         const int nsolves = nsolves_;
@@ -608,7 +621,7 @@ int EngineT<Real>::autotune_resident(size_t ncand) {
         }
         use(besti);
     }
-    tuned_resident_[key] = blk_;
+    tuned_resident_[key] = plan_at_;
     return TOMO_OK;
 }
 
@@ -771,7 +784,7 @@ template <typename Real>
 int EngineT<Real>::build_graph(int nlaunch) {
     const bool resident = blk_.blocks > 0;
     if (graph_exec_ && graph_cand_ == cur_cand_ && graph_blk_ == blk_ && graph_launches_ == nlaunch &&
-        (!resident || (graph_smem_ == plan_batch_[plan_at_].smem && graph_warps_ == plan_batch_[plan_at_].warps)))
+        (!resident || graph_batch_ == launch_key(plan_batch_[plan_at_])))
         return TOMO_OK;
     invalidate_graph();
     int blocks = 0, clusters = 0;
@@ -815,10 +828,7 @@ int EngineT<Real>::build_graph(int nlaunch) {
         return fail(TOMO_ECUDA, std::string("graph instantiate: ") + cudaGetErrorString(ce));
     }
     graph_cand_ = cur_cand_; graph_blk_ = blk_; graph_launches_ = nlaunch; graph_blocks_ = blocks;
-    if (resident) {
-        graph_smem_ = plan_batch_[plan_at_].smem;
-        graph_warps_ = plan_batch_[plan_at_].warps;
-    }
+    if (resident) graph_batch_ = launch_key(plan_batch_[plan_at_]);
     return TOMO_OK;
 }
 
@@ -832,12 +842,8 @@ int EngineT<Real>::forward(const double* args, size_t ncand, size_t nparam, cons
     stats_.tune_ms = 0;
     stats_.tuned_configs = 0;
     bool fits = false;
-    for (size_t i = 0; i < plans_.size(); ++i) {
-        resident_batch<Real>(pc, plans_[i], up_, plan_batch_[i]);
-        fits |= plan_batch_[i].fits;
-    }
+    TOMO_TRY(pick_resident(ncand, &fits));
     if (fits) {
-        TOMO_TRY(autotune_resident(ncand));
     } else if ((auto_T_ || auto_cols_ || auto_minb_) && !s.plain) {
         auto it = tuned_.find((int)ncand * pc.n_exc);
         if (it != tuned_.end()) {

@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstdint>
 #include <cstdlib>
@@ -420,11 +421,21 @@ struct ResidentPlan {
 // A batch on a plan: every candidate's slabs, and what a launch needs.
 struct ResidentBatch {
     bool fits = false;
+    ResidentShape shape{0, 0};
     int warps = 0;             // per block
     size_t smem = 0;           // per block
     std::vector<int> ys;       // [ncand (+ 1)][blocks + 1]: first row of each slab, then ny
-    double cost = 0;           // of the dearest slab
+    double cost = 0;           // of the dearest slab: about its microseconds a step past 0.9
 };
+inline std::array<size_t, 4> launch_key(const ResidentBatch& b) {
+    return {b.smem, (size_t)b.warps, (size_t)b.shape.share, (size_t)b.shape.warps};
+}
+// Blocks per cluster on offer: of the sizes with as many clusters on the GPU the largest.
+constexpr int kClusterSizes[] = {16, 12, 10, 9, 6, 5, 4};
+// About the microseconds of a time step of nsolves solves.
+inline double resident_estimate(const ResidentBatch& b, int nsolves, int clusters) {
+    return ((nsolves + clusters - 1) / clusters) * (0.9 + b.cost);
+}
 // false: the class does not fit the resident kernel with that many blocks.
 template <typename Real>
 bool resident_plan(const ProblemClass& pc, const SolveLayout& lay, int blocks, ResidentPlan& p);
@@ -631,7 +642,7 @@ class EngineT : public EngineBase {
     int ensure_batch(int ncand);
     int build_graph(int nlaunch);
     int autotune(size_t ncand);
-    int autotune_resident(size_t ncand);
+    int pick_resident(size_t ncand, bool* fits);
     int upload_descs(size_t ncand);
     void invalidate_graph() {
         if (graph_exec_) cudaGraphExecDestroy(graph_exec_);
@@ -651,12 +662,11 @@ class EngineT : public EngineBase {
     bool auto_T_ = false, auto_cols_ = false, auto_minb_ = false;   // tuned per batch size on first use
     int fix_T_ = 0, fix_cols_ = 0, fix_minb_ = 0;  // dimensions fixed by the spec or the environment
     std::map<int, Blocking> tuned_;                // solves per batch -> blocking
-    std::map<int, Blocking> tuned_resident_;       // the same among the resident plans
+    std::map<int, size_t> tuned_resident_;         // solves per batch -> resident plan
     std::vector<ResidentPlan> plans_;              // resident plans of the class, most blocks first
     std::vector<ResidentBatch> plan_batch_;        // the current batch on each
     size_t plan_at_ = 0;                           // the one of blk_ when blk_.blocks > 0
-    size_t graph_smem_ = 0;
-    int graph_warps_ = 0;
+    std::array<size_t, 4> graph_batch_{};          // what the captured launch was made for
     Blocking items_blk_{-1, -1, -1};               // blocking the uploaded work items were cut for
     DevBuf d_tune_items_;
     uint64_t budget_ = (uint64_t)150 << 30;

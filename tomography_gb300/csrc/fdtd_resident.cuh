@@ -36,11 +36,10 @@
 namespace tomo {
 
 constexpr int kEdge = 16;            // columns of either side in the edge pass (ncpml <= kEdge - 1)
-constexpr int kRows = 4;             // rows per warp
-// Most warps of a block by the number of inner passes: the fields of a warp's rows
-// fill the registers, of which 8 warps leave 255 a thread and 12 leave 168.
-constexpr int resident_warps(int passes) { return passes == 1 ? 12 : 8; }
-constexpr int kResidentWarps = 12;
+constexpr int kRows = 4;             // most rows per warp
+constexpr int kResidentWarps = 16;   // most warps per block
+// The edge pass takes rows in pairs.
+__host__ __device__ constexpr int resident_even(int share) { return (share + 1) / 2 * 2; }
 
 // 16 bytes of a row: the columns of one lane in a pass.
 template <typename Real>
@@ -191,10 +190,10 @@ struct ResidentLayout {
     size_t jp, gp, ejp, psy, psx, prof, cpml, tab, tab2, hf, rx, warps, samp, points, mats, emats, total;
 };
 
-// rows: the slab [ya, yb); maxrow: the tallest slab of the cluster.
+// share: rows per warp; [ya, yb): the slab; maxrow: the tallest slab of the cluster.
 template <typename Real>
 __host__ __device__ inline ResidentLayout resident_layout(int nx, int ny, int nc, int nmat, bool ref, int passes,
-                                                          int ya, int yb, int maxrow, int mx0, int mx1, int my0,
+                                                          int share, int ya, int yb, int maxrow, int mx0, int mx1, int my0,
                                                           int my1, int d) {
     ResidentLayout L{};
     if (d >= 0) {   // NTFF distance, -1: none
@@ -204,8 +203,8 @@ __host__ __device__ inline ResidentLayout resident_layout(int nx, int ny, int nc
         if (ny - d - 1 >= ya && ny - d - 1 < yb) L.npoints += nx - 2 * d - 2;
     }
     L.pitch = passes * 32 * Quad<Real>::N + 2 * kEdge;
-    L.ez_rows = maxrow + kRows + 1;
-    const int warps = (yb - ya + kRows - 1) / kRows;
+    L.ez_rows = maxrow + share + 1;
+    const int warps = (yb - ya + share - 1) / share;
     L.br0 = my0 > ya ? my0 : ya;
     L.br1 = my1 + 1 < yb ? my1 + 1 : yb;
     const int right = resident_right<Real>(nx);
@@ -222,9 +221,9 @@ __host__ __device__ inline ResidentLayout resident_layout(int nx, int ny, int nc
     L.psi_hi = warps;
     if (nc > 0)
         for (int w = 0; w < warps; ++w) {
-            const int y0 = ya + kRows * w;
+            const int y0 = ya + share * w;
             if (y0 - 1 <= nc) L.psi_lo = w + 1;
-            if (y0 + kRows - 1 >= ny - nc && L.psi_hi == warps) L.psi_hi = w;
+            if (y0 + share - 1 >= ny - nc && L.psi_hi == warps) L.psi_hi = w;
         }
     if (L.psi_hi < L.psi_lo) L.psi_hi = L.psi_lo;
     const int npsi = L.psi_lo + (warps - L.psi_hi);
@@ -238,8 +237,8 @@ __host__ __device__ inline ResidentLayout resident_layout(int nx, int ny, int nc
     L.jp = take(sizeof(Real) * cells);
     L.gp = take(ref ? sizeof(Real) * (size_t)brows * bw : 0);
     L.ejp = take(L.edge_mat ? sizeof(Real) * (size_t)brows * 32 : 0);
-    L.psy = take(sizeof(Real) * (size_t)npsi * (2 * kRows + 1) * L.pitch);
-    L.psx = take(nc > 0 ? sizeof(Real) * (size_t)warps * 2 * kRows * 32 : 0);
+    L.psy = take(sizeof(Real) * (size_t)npsi * (2 * share + 1) * L.pitch);
+    L.psx = take(nc > 0 ? sizeof(Real) * (size_t)warps * 2 * resident_even(share) * 32 : 0);
     L.prof = take(sizeof(Real) * 8 * 32);
     L.cpml = take(sizeof(Real) * 6 * nc);
     L.tab = take(sizeof(Real) * 4 * (size_t)nmat);
@@ -296,10 +295,10 @@ __device__ __forceinline__ Real plane_front(const ResidentWarp<Real>& w, double 
 // y0 .. y0 + kRows - 1.  hx: from row y0-1; hy: from row y0; cur points at Ez(x, y0) of the
 // step's old copy, nxt at the new one; left: Hy of the column before the pass
 // (valid in lane 31).  YP: y-CPML rows; MAT: materials; both: the source too.
-template <typename Real, int P, int MODE, bool YP, bool MAT, bool LAST>
+template <typename Real, int P, int MODE, int R, bool YP, bool MAT, bool LAST>
 __device__ __forceinline__ void resident_pass(const ResidentWarp<Real>& w, const ResidentHot<Real>& g,
-                                              Quad<Real> (&hx)[kRows + 1], Quad<Real> (&hy)[kRows],
-                                              const Real (&left)[kRows],
+                                              Quad<Real> (&hx)[R + 1], Quad<Real> (&hy)[R],
+                                              const Real (&left)[resident_even(R)],
                                               const Real* cur, Real* nxt, int x) {
     using O = Op<Real>;
     constexpr int N = Quad<Real>::N;
@@ -307,17 +306,17 @@ __device__ __forceinline__ void resident_pass(const ResidentWarp<Real>& w, const
     const Two<Real> chez2 = dup2<Real>(g.chez), mchez2 = dup2<Real>(-g.chez);
     const int end = g.end;   // the columns from here on belong to the edge pass
     const int lane = threadIdx.x & 31;
-    Quad<Real> e[kRows + 2];   // Ez rows from y0-1
+    Quad<Real> e[R + 2];   // Ez rows from y0-1
 #pragma unroll
-    for (int i = 0; i < kRows + 2; ++i) e[i] = ldq<Real>(cur + (i - 1) * P);
+    for (int i = 0; i < R + 2; ++i) e[i] = ldq<Real>(cur + (i - 1) * P);
     // materials and Debye current of the rows, loaded ahead of the first store
-    Quad<Real> jp[kRows] = {}, gm[kRows] = {};
-    uint32_t mb[kRows] = {};
-    bool in[kRows] = {};
-    int at[kRows] = {};
+    Quad<Real> jp[R] = {}, gm[R] = {};
+    uint32_t mb[R] = {};
+    bool in[R] = {};
+    int at[R] = {};
     if constexpr (MAT) {
 #pragma unroll
-        for (int j = 0; j < kRows; ++j) {
+        for (int j = 0; j < R; ++j) {
             // lanes outside the box read its first cells and drop them
             in[j] = w.jr[j] >= 0 && x >= w.bx0 && x < w.bx1;
             at[j] = in[j] ? w.jr[j] * (w.bx1 - w.bx0) + x - w.bx0 : 0;
@@ -333,16 +332,16 @@ __device__ __forceinline__ void resident_pass(const ResidentWarp<Real>& w, const
     }
     // y-CPML psi of the rows, likewise
     constexpr bool kStrip = YP && !MAT;
-    Quad<Real> psh[kRows + 1], pse[kRows];
+    Quad<Real> psh[R + 1], pse[R];
     if constexpr (kStrip) {
 #pragma unroll
-        for (int r = 0; r < kRows + 1; ++r) psh[r] = ldq<Real>(shared_at<Real>(w.psy) + r * P + x);
+        for (int r = 0; r < R + 1; ++r) psh[r] = ldq<Real>(shared_at<Real>(w.psy) + r * P + x);
 #pragma unroll
-        for (int j = 0; j < kRows; ++j) pse[j] = ldq<Real>(shared_at<Real>(w.psy) + (kRows + 1 + j) * P + x);
+        for (int j = 0; j < R; ++j) pse[j] = ldq<Real>(shared_at<Real>(w.psy) + (R + 1 + j) * P + x);
     }
     // H update
 #pragma unroll
-    for (int j = 0; j < kRows; ++j) {
+    for (int j = 0; j < R; ++j) {
         Real er = __shfl_down_sync(0xffffffffu, e[j + 1].v[0], 1);
         if (lane == 31) er = cur[j * P + N];
 #pragma unroll
@@ -357,7 +356,7 @@ __device__ __forceinline__ void resident_pass(const ResidentWarp<Real>& w, const
         if (kRef && g.clampnan) clamp_nans(hy[j].v);
     }
 #pragma unroll
-    for (int r = 0; r < kRows + 1; ++r) {
+    for (int r = 0; r < R + 1; ++r) {
         const int iy = YP && MAT ? w.iyh[r] : -1;
         if constexpr (kStrip) {
             Real b, a, rk, flag;
@@ -399,9 +398,9 @@ __device__ __forceinline__ void resident_pass(const ResidentWarp<Real>& w, const
         if (kRef && g.clampnan) clamp_nans(hx[r].v);
     }
     // E update
-    Quad<Real> out[kRows], jn[kRows];
+    Quad<Real> out[R], jn[R];
 #pragma unroll
-    for (int j = 0; j < kRows; ++j) {
+    for (int j = 0; j < R; ++j) {
         const Real hv = lane == 31 ? left[j] : hy[j].v[N - 1];
         const Real hl = __shfl_sync(0xffffffffu, hv, (lane + 31) & 31);
         const int iy = YP && MAT ? w.iye[j] : -1;
@@ -438,7 +437,7 @@ __device__ __forceinline__ void resident_pass(const ResidentWarp<Real>& w, const
                 out[j].v[2 * i] = t.x;
                 out[j].v[2 * i + 1] = t.y;
             }
-            if constexpr (kStrip) stq_until<LAST>(shared_at<Real>(w.psy) + (kRows + 1 + j) * P + x, pse[j], x, end);
+            if constexpr (kStrip) stq_until<LAST>(shared_at<Real>(w.psy) + (R + 1 + j) * P + x, pse[j], x, end);
         } else {
             Quad<Real> gp{};
             if (in[j]) {
@@ -457,7 +456,7 @@ __device__ __forceinline__ void resident_pass(const ResidentWarp<Real>& w, const
             if (YP && iy >= 0) {
                 const Real b = shared_at<Real>(w.cpml)[w.nc + iy], a = shared_at<Real>(w.cpml)[2 * w.nc + iy];
                 rk = shared_at<Real>(w.cpml)[iy];
-                Real* pp = shared_at<Real>(w.psy) + (kRows + 1 + j) * P + x;
+                Real* pp = shared_at<Real>(w.psy) + (R + 1 + j) * P + x;
                 psn = ldq<Real>(pp);
 #pragma unroll
                 for (int i = 0; i < N; ++i)
@@ -494,7 +493,7 @@ __device__ __forceinline__ void resident_pass(const ResidentWarp<Real>& w, const
     }
     // stores last: the loads of a row need not wait for the row before
 #pragma unroll
-    for (int j = 0; j < kRows; ++j) {
+    for (int j = 0; j < R; ++j) {
         if (j < g.nr) stq_until<LAST>(nxt + j * P, out[j], x, end);
         if (MAT && in[j]) stq<Real>(shared_at<Real>(w.jp) + at[j], jn[j]);
     }
@@ -508,20 +507,20 @@ __device__ __forceinline__ void resident_pass(const ResidentWarp<Real>& w, const
 // update's bits as they are, the magnetic one is chosen by select.  hyl: Hy of
 // column xq (nx - 16, lane 16's left neighbour), kept redundantly.  YP: y-CPML
 // rows; ALL: materials and the source too.
-template <typename Real, int P, int MODE, bool YP, bool ALL>
+template <typename Real, int P, int MODE, int R, bool YP, bool ALL>
 __device__ __forceinline__ void resident_edge(const ResidentWarp<Real>& w, const ResidentHot<Real>& g,
-                                              Real (&hx)[kRows + 1], Two<Real> (&hy)[kRows / 2],
-                                              Two<Real> (&hyl)[kRows / 2], const Real* cur, Real* nxt, int xe, int xq,
+                                              Real (&hx)[resident_even(R) + 1], Two<Real> (&hy)[(R + 1) / 2],
+                                              Two<Real> (&hyl)[(R + 1) / 2], const Real* cur, Real* nxt, int xe, int xq,
                                               bool isxh, bool isxe, Real* psx, const Real* prof, bool cpml, bool mats,
                                               Real* ejp, const uint8_t* emats) {
     using O = Op<Real>;
     constexpr bool kRef = MODE == kModeRef;
-    constexpr int kPairs = kRows / 2;
+    constexpr int kPairs = (R + 1) / 2;
     const int lane = threadIdx.x & 31;
     const bool mine = lane < kEdge || xe >= g.end;   // else an inner column: nothing of it is written here
-    Real e[kRows + 2];
+    Real e[R + 2];
 #pragma unroll
-    for (int i = 0; i < kRows + 2; ++i) e[i] = cur[xe + (i - 1) * P];
+    for (int i = 0; i < R + 2; ++i) e[i] = cur[xe + (i - 1) * P];
     const Two<Real> chez2 = dup2<Real>(g.chez), ca = dup2<Real>(g.Ca0), cb = dup2<Real>(g.Cb0);
     Real rke, be, ae, rkm, bm, am, unused;
     load_coefs(prof, rke, be, ae, unused);
@@ -531,16 +530,16 @@ __device__ __forceinline__ void resident_edge(const ResidentWarp<Real>& w, const
 #pragma unroll
         for (int q = 0; q < kPairs; ++q) {
             ph[q] = *reinterpret_cast<const Two<Real>*>(psx + 2 * q);
-            pe[q] = *reinterpret_cast<const Two<Real>*>(psx + kRows + 2 * q);
+            pe[q] = *reinterpret_cast<const Two<Real>*>(psx + 2 * kPairs + 2 * q);
         }
     }
-    Real psh[kRows + 1] = {}, pse[kRows] = {};
+    Real psh[R + 1] = {}, pse[2 * kPairs] = {};
     if constexpr (YP) {
         const Real* const psy = shared_at<Real>(w.psy) + xe;
 #pragma unroll
-        for (int r = 0; r < kRows + 1; ++r) psh[r] = psy[r * P];
+        for (int r = 0; r < R + 1; ++r) psh[r] = psy[r * P];
 #pragma unroll
-        for (int j = 0; j < kRows; ++j) pse[j] = psy[(kRows + 1 + j) * P];
+        for (int j = 0; j < R; ++j) pse[j] = psy[(R + 1 + j) * P];
     }
     // Hy
 #pragma unroll
@@ -555,7 +554,7 @@ __device__ __forceinline__ void resident_edge(const ResidentWarp<Real>& w, const
     }
     // Hx from row y0-1
 #pragma unroll
-    for (int r = 0; r < kRows + 1; ++r) {
+    for (int r = 0; r < R + 1; ++r) {
         const Real dEx = O::sub(e[r + 1], e[r]), plain = O::fma(-g.chez, dEx, hx[r]);
         if constexpr (YP) {
             Real b, a, rk, on;
@@ -568,7 +567,7 @@ __device__ __forceinline__ void resident_edge(const ResidentWarp<Real>& w, const
         }
     }
     if (kRef && g.clampnan) {
-        Real v[2 * kRows];
+        Real v[4 * kPairs];
 #pragma unroll
         for (int q = 0; q < kPairs; ++q) {
             v[4 * q] = hy[q].x; v[4 * q + 1] = hy[q].y; v[4 * q + 2] = hyl[q].x; v[4 * q + 3] = hyl[q].y;
@@ -643,15 +642,15 @@ __device__ __forceinline__ void resident_edge(const ResidentWarp<Real>& w, const
 #pragma unroll
         for (int q = 0; q < kPairs; ++q) {
             *reinterpret_cast<Two<Real>*>(psx + 2 * q) = ph[q];
-            *reinterpret_cast<Two<Real>*>(psx + kRows + 2 * q) = pe[q];
+            *reinterpret_cast<Two<Real>*>(psx + 2 * kPairs + 2 * q) = pe[q];
         }
     }
     if (YP && mine) {
         Real* const psy = shared_at<Real>(w.psy) + xe;
 #pragma unroll
-        for (int r = 0; r < kRows + 1; ++r) psy[r * P] = psh[r];
+        for (int r = 0; r < R + 1; ++r) psy[r * P] = psh[r];
 #pragma unroll
-        for (int j = 0; j < kRows; ++j) psy[(kRows + 1 + j) * P] = pse[j];
+        for (int j = 0; j < R; ++j) psy[(R + 1 + j) * P] = pse[j];
     }
 }
 
@@ -661,7 +660,7 @@ __device__ __forceinline__ void resident_edge(const ResidentWarp<Real>& w, const
 template <typename Real, int P>
 __device__ __forceinline__ void resident_sample(const ResidentSampler<Real>& q, const int* rx,
                                                 const ResidentPoint* points, const Real* nxt, const Real* h, int k) {
-    const int t = threadIdx.x;
+    const int t = blockDim.x - 1 - threadIdx.x;   // the last warps first: they may have no rows
     if (t < q.nrx && rx[t] >= 0) q.traces[(size_t)t * q.S + k] = nxt[rx[t]];
     for (int i = t; i < q.total; i += blockDim.x) {
         const ResidentPoint p = points[i];
@@ -689,12 +688,13 @@ enum ResidentTodo : unsigned {
 // alternate copies).  The contour samples of step D.step + k go to staging
 // level k.  *error is set when a halo row did not arrive.  The sampler reads Ez
 // of the row above a horizontal NTFF face from the same block: no slab ends at one.
-template <typename Real, int PASSES, int MODE>
-__global__ void __launch_bounds__(32 * resident_warps(PASSES), 1)
+template <typename Real, int PASSES, int MODE, int R, int W>
+__global__ void __launch_bounds__(32 * W, 1)
     fdtd_resident_kernel(const SolveDesc<Real>* __restrict__ descs, int nsolves, int nsteps, int* __restrict__ error) {
     extern __shared__ __align__(16) unsigned char smem[];
     constexpr int N = Quad<Real>::N, P = 32 * N * PASSES + 2 * kEdge;
     constexpr bool kRef = MODE == kModeRef;
+    constexpr int kEven = resident_even(R);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int rank = (int)cluster_rank(), nblk = (int)cluster_blocks();
     const int nclusters = gridDim.x / nblk;
@@ -711,7 +711,7 @@ __global__ void __launch_bounds__(32 * resident_warps(PASSES), 1)
         const int ya = D.ys[rank], yb = D.ys[rank + 1];
         int maxrow = 0;
         for (int b = 0; b < nblk; ++b) maxrow = max(maxrow, D.ys[b + 1] - D.ys[b]);
-        const ResidentLayout L = resident_layout<Real>(nx, ny, nc, D.nmat, kRef, PASSES, ya, yb, maxrow, D.mx0, D.mx1,
+        const ResidentLayout L = resident_layout<Real>(nx, ny, nc, D.nmat, kRef, PASSES, R, ya, yb, maxrow, D.mx0, D.mx1,
                                                        D.my0, D.my1, D.nfreq > 0 ? D.nf_d : -1);
         const int pitch = D.pitch;
         Real* const ez_s = reinterpret_cast<Real*>(smem + kBarBytes);
@@ -824,11 +824,11 @@ __global__ void __launch_bounds__(32 * resident_warps(PASSES), 1)
 
         // ---- the warp's rows
         ResidentWarp<Real>& w = reinterpret_cast<ResidentWarp<Real>*>(smem + L.warps)[warp];
-        const int y0 = ya + kRows * warp, l0 = y0 - ya + 1, nr = max(0, min(kRows, yb - y0));
+        const int y0 = ya + R * warp, l0 = y0 - ya + 1, nr = max(0, min(R, yb - y0));
         w.nc = nc;   // every lane writes the same values
         bool ypml = false;
 #pragma unroll
-        for (int r = 0; r < kRows + 1; ++r) {
+        for (int r = 0; r < R + 1; ++r) {
             const int m = y0 - 1 + r;
             w.iyh[r] = m < nc ? nc - 1 - m : ((m >= ny - nc && m < ny) ? m - ny + nc : -1);
             ypml |= w.iyh[r] >= 0;
@@ -836,11 +836,11 @@ __global__ void __launch_bounds__(32 * resident_warps(PASSES), 1)
 #pragma unroll
         for (int j = 0; j < kRows; ++j) {
             const int m = y0 + j;
-            w.iye[j] = m <= nc ? nc - m : ((m >= ny - nc && m <= ny - 1) ? m - ny + nc : -1);
+            w.iye[j] = j >= R ? -1 : m <= nc ? nc - m : ((m >= ny - nc && m <= ny - 1) ? m - ny + nc : -1);
             ypml |= w.iye[j] >= 0;
-            w.jr[j] = (m >= L.br0 && m < L.br1) ? m - L.br0 : -1;
+            w.jr[j] = (j < R && m >= L.br0 && m < L.br1) ? m - L.br0 : -1;
             const bool valid = j < nr;
-w.src[j] = -1;
+            w.src[j] = -1;
             w.hface[j] = (D.nfreq > 0 && valid) ? (m == D.nf_d ? 0 : (m == ny - D.nf_d - 1 ? 1 : -1)) : -1;
         }
         w.bx0 = L.bx0;
@@ -864,9 +864,9 @@ w.src[j] = -1;
         w.mats = (int)L.mats;
         w.cs = w.wave = Real(0);
         const int slot = warp < L.psi_lo ? warp : warp - L.psi_hi + L.psi_lo;
-        w.psy = (int)(L.psy + sizeof(Real) * (size_t)slot * (2 * kRows + 1) * P);
+        w.psy = (int)(L.psy + sizeof(Real) * (size_t)slot * (2 * R + 1) * P);
         Real* const psy = shared_at<Real>(w.psy);
-        Real* const psx = psx_s + ((size_t)warp * 32 + lane) * 2 * kRows;
+        Real* const psx = psx_s + ((size_t)warp * 32 + lane) * 2 * kEven;
         const bool has_src = (D.flags & kPointSource) && D.src_y >= y0 && D.src_y < y0 + nr;
         // a source in the background is added to the finished row; among materials (the Debye
         // current takes it in) or in a strip of the reference modes the general passes do it
@@ -876,7 +876,7 @@ w.src[j] = -1;
             w.cs = D.mtab[mat * kMatCoef + kCs];
             src_all = mat != 0 || kRef;
 #pragma unroll
-            for (int j = 0; j < kRows; ++j)
+            for (int j = 0; j < R; ++j)
                 if (src_all && y0 + j == D.src_y) w.src[j] = D.src_x;
         }
         w.plane = kRef && (D.flags & kPlaneWave) != 0;
@@ -886,7 +886,7 @@ w.src[j] = -1;
             w.pw_dxc0 = D.pw_dxc0;
             w.pw_inv_tau = D.pw_inv_tau;
 #pragma unroll
-            for (int j = 0; j < kRows; ++j) {
+            for (int j = 0; j < R; ++j) {
                 w.pw_row[j] = __dmul_rn(D.pw_ky, (double)(y0 + j) - D.pw_yoff);
                 w.pwf_row[j] = (float)(w.pw_row[j] * D.pw_dxc0 * D.pw_inv_tau);
             }
@@ -897,14 +897,14 @@ w.src[j] = -1;
             w.pwf_reach = (sizeof(Real) == 8 ? 27.6f : 10.5f) + N * fabsf(w.pwf_col) +
                           1e-5f * (float)(D.pw_inv_tau * (S * D.dt + fabs(D.pw_t0l) + (nx + ny) * D.pw_dxc0));
         }
-        if (lane < kRows + 1) {
+        if (lane < R + 1) {
             const int iy = w.iyh[lane];
             w.hc[lane][0] = iy >= 0 ? D.cpml[4 * nc + iy] : Real(0);
             w.hc[lane][1] = iy >= 0 ? D.cpml[5 * nc + iy] : Real(0);
             w.hc[lane][2] = iy >= 0 ? D.cpml[3 * nc + iy] : Real(1);
             w.hc[lane][3] = iy >= 0 ? Real(1) : Real(0);
-        } else if (lane < 2 * kRows + 1) {
-            const int at = lane - kRows - 1, iy = w.iye[at];
+        } else if (lane < 2 * R + 1) {
+            const int at = lane - R - 1, iy = w.iye[at];
             w.ec[at][0] = iy >= 0 ? D.cpml[nc + iy] : Real(0);
             w.ec[at][1] = iy >= 0 ? D.cpml[2 * nc + iy] : Real(0);
             w.ec[at][2] = iy >= 0 ? D.cpml[iy] : Real(1);
@@ -914,7 +914,7 @@ w.src[j] = -1;
         // passes with materials, and with a source that the pass adds
         bool box_rows = false;
 #pragma unroll
-        for (int j = 0; j < kRows; ++j) box_rows |= w.jr[j] >= 0;
+        for (int j = 0; j < R; ++j) box_rows |= w.jr[j] >= 0;
         unsigned matmask = 0, srcmask = 0;
 #pragma unroll
         for (int c = 0; c < PASSES; ++c) {
@@ -940,13 +940,13 @@ w.src[j] = -1;
         if (from_below) todo |= kBelow;
         if (from_above) todo |= kAbove;
 #pragma unroll
-        for (int j = 0; j < kRows; ++j)
+        for (int j = 0; j < R; ++j)
             if (w.hface[j] >= 0) todo |= kFaceRow;
         if (nfaces) todo |= kFaceColumns;
         if (has_src) todo |= kSource;
         if (has_src && !src_all) todo |= kSourceAdd;
         if (kRef && (D.flags & kPlaneWave)) todo |= kPlane;
-        if (32 * warp < max(L.npoints, (int)D.nrx)) todo |= kSample;
+        if (32 * (nwarp - 1 - warp) < max(L.npoints, (int)D.nrx)) todo |= kSample;
         todo = __reduce_or_sync(0xffffffffu, todo);
 
         // column whose Hy ehyl follows: the left neighbour of lane 16, and in lanes 0 and 1
@@ -954,9 +954,9 @@ w.src[j] = -1;
         const int xq = nfaces && lane < 2 ? (lane ? nx - D.nf_d - 1 : D.nf_d) : nx - kEdge;
 
         // fields of the warp's rows
-        Quad<Real> hx[PASSES][kRows + 1], hy[PASSES][kRows];
-        Real ehx[kRows + 1];
-        Two<Real> ehy[kRows / 2] = {}, ehyl[kRows / 2] = {};
+        Quad<Real> hx[PASSES][R + 1], hy[PASSES][R];
+        Real ehx[kEven + 1] = {};
+        Two<Real> ehy[kEven / 2] = {}, ehyl[kEven / 2] = {};
         // Hx and Hy are zero from column nx and row ny on, in memory too
         const Real *const hx_g = D.hx[0], *const hy_g = D.hy[0];
         auto row_of = [&](const Real* f, int m) { return f + (size_t)min(m, ny) * pitch; };
@@ -965,37 +965,37 @@ w.src[j] = -1;
             for (int c = 0; c < PASSES; ++c) {
                 const int x = kEdge + 32 * N * c + N * lane;
 #pragma unroll
-                for (int r = 0; r < kRows + 1; ++r) hx[c][r] = n0 > 0 ? ldq<Real>(row_of(hx_g, y0 - 1 + r) + x) : Quad<Real>{};
+                for (int r = 0; r < R + 1; ++r) hx[c][r] = n0 > 0 ? ldq<Real>(row_of(hx_g, y0 - 1 + r) + x) : Quad<Real>{};
 #pragma unroll
-                for (int j = 0; j < kRows; ++j) hy[c][j] = n0 > 0 ? ldq<Real>(row_of(hy_g, y0 + j) + x) : Quad<Real>{};
+                for (int j = 0; j < R; ++j) hy[c][j] = n0 > 0 ? ldq<Real>(row_of(hy_g, y0 + j) + x) : Quad<Real>{};
             }
 #pragma unroll
-            for (int r = 0; r < kRows + 1; ++r) ehx[r] = row_of(hx_g, y0 - 1 + r)[xe];
+            for (int r = 0; r < R + 1; ++r) ehx[r] = row_of(hx_g, y0 - 1 + r)[xe];
 #pragma unroll
-            for (int q = 0; q < kRows / 2; ++q) {
+            for (int q = 0; q < kEven / 2; ++q) {
                 ehy[q] = {row_of(hy_g, y0 + 2 * q)[xe], row_of(hy_g, y0 + 2 * q + 1)[xe]};
                 ehyl[q] = {row_of(hy_g, y0 + 2 * q)[xq], row_of(hy_g, y0 + 2 * q + 1)[xq]};
             }
             if (nc > 0) {
                 const int xh = xe < nc ? xe : xe - (nx - nc) + nc, xq = xe <= nc ? xe - 1 : xe - (nx - nc) + nc;
 #pragma unroll
-                for (int j = 0; j < kRows; ++j) {
+                for (int j = 0; j < R; ++j) {
                     const int m = y0 + j;
                     psx[j] = (ixh >= 0 && m < ny) ? psi_g[psx_h + (size_t)m * 2 * nc + xh] : Real(0);
-                    psx[kRows + j] = (ixe >= 0 && m < ny) ? psi_g[psx_e + (size_t)m * 2 * nc + xq] : Real(0);
+                    psx[kEven + j] = (ixe >= 0 && m < ny) ? psi_g[psx_e + (size_t)m * 2 * nc + xq] : Real(0);
                 }
             }
             if (ypml)
                 for (int x = lane; x < P; x += 32) {
 #pragma unroll
-                    for (int r = 0; r < kRows + 1; ++r) {
+                    for (int r = 0; r < R + 1; ++r) {
                         const int m = y0 - 1 + r, yh = m < nc ? m : m - (ny - nc) + nc;
                         psy[r * P + x] = (w.iyh[r] >= 0 && x < nx) ? psi_g[psy_h + (size_t)yh * (nx + 1) + x] : Real(0);
                     }
 #pragma unroll
-                    for (int j = 0; j < kRows; ++j) {
+                    for (int j = 0; j < R; ++j) {
                         const int m = y0 + j, ye = m <= nc ? m - 1 : m - (ny - nc) + nc;
-                        psy[(kRows + 1 + j) * P + x] =
+                        psy[(R + 1 + j) * P + x] =
                             (w.iye[j] >= 0 && x >= 1 && x <= nx - 1) ? psi_g[psy_e + (size_t)ye * (nx + 1) + x] : Real(0);
                     }
                 }
@@ -1005,7 +1005,7 @@ w.src[j] = -1;
             // the front of the previous half step, which every later step takes over
             const double t1 = __dsub_rn(__dmul_rn((double)n0 - 0.5, D.dt), D.pw_t0l);
 #pragma unroll
-            for (int j = 0; j < kRows; ++j)
+            for (int j = 0; j < R; ++j)
                 if (w.jr[j] >= 0 && j < nr)
                     for (int i = lane; i < bw; i += 32) gp_s[w.jr[j] * bw + i] = plane_front(w, t1, j, L.bx0 + i);
         }
@@ -1056,16 +1056,16 @@ w.src[j] = -1;
                 const Real* const rowc = cur + l0 * P;
                 Real* const rown = nxt + l0 * P;
 #define TOMO_EDGE(YP, ALL)                                                                                       \
-    resident_edge<Real, P, MODE, YP, ALL>(w, g, ehx, ehy, ehyl, rowc, rown, xe, xq, ixh >= 0, ixe >= 0, psx,     \
+    resident_edge<Real, P, MODE, R, YP, ALL>(w, g, ehx, ehy, ehyl, rowc, rown, xe, xq, ixh >= 0, ixe >= 0, psx,     \
                                           prof_s + 8 * lane, cpml, L.edge_mat != 0, ejp_s, emats_s)
                 if ((todo & kEdgeAll) && (todo & kEdgeStrip)) TOMO_EDGE(true, true);
                 else if (todo & kEdgeAll) TOMO_EDGE(false, true);
                 else if (todo & kEdgeStrip) TOMO_EDGE(true, false);
                 else TOMO_EDGE(false, false);
 #undef TOMO_EDGE
-                Real left[kRows];
+                Real left[kEven];
 #pragma unroll
-                for (int q = 0; q < kRows / 2; ++q) {
+                for (int q = 0; q < kEven / 2; ++q) {
                     left[2 * q] = __shfl_sync(0xffffffffu, ehy[q].x, 15);
                     left[2 * q + 1] = __shfl_sync(0xffffffffu, ehy[q].y, 15);
                 }
@@ -1077,9 +1077,9 @@ w.src[j] = -1;
 #define TOMO_PASS(YP, MAT)                                                                                    \
     do {                                                                                                      \
         if (c == kLast)                                                                                       \
-            resident_pass<Real, P, MODE, YP, MAT, true>(w, g, hx[c], hy[c], left, rowc + x, rown + x, x); \
+            resident_pass<Real, P, MODE, R, YP, MAT, true>(w, g, hx[c], hy[c], left, rowc + x, rown + x, x); \
         else                                                                                                  \
-            resident_pass<Real, P, MODE, YP, MAT, false>(w, g, hx[c], hy[c], left, rowc + x, rown + x, x); \
+            resident_pass<Real, P, MODE, R, YP, MAT, false>(w, g, hx[c], hy[c], left, rowc + x, rown + x, x); \
     } while (0)
                     if (kind == kPassAll) TOMO_PASS(true, true);
                     else if (kind == kPassStrip) TOMO_PASS(true, false);
@@ -1087,7 +1087,7 @@ w.src[j] = -1;
                     else TOMO_PASS(false, false);
 #undef TOMO_PASS
 #pragma unroll
-                    for (int j = 0; j < kRows; ++j) left[j] = hy[c][j].v[N - 1];
+                    for (int j = 0; j < R; ++j) left[j] = hy[c][j].v[N - 1];
                 }
                 if (todo & kSourceAdd) {
                     __syncwarp();
@@ -1099,7 +1099,7 @@ w.src[j] = -1;
                 // H of the NTFF faces for the sampler: Hx of the face rows, Hy of the face columns
                 if (todo & kFaceRow) {
 #pragma unroll
-                    for (int j = 0; j < kRows; ++j)
+                    for (int j = 0; j < R; ++j)
                         if (w.hface[j] >= 0) {
                             Real* const o = hf_s + (k & 1) * L.hstep + w.hface[j] * P;
 #pragma unroll
@@ -1114,7 +1114,7 @@ w.src[j] = -1;
                 if ((todo & kFaceColumns) && lane < 2) {
                     Real* const o = hf_s + (k & 1) * L.hstep + 2 * P + 2 * (y0 - ya) + lane;
 #pragma unroll
-                    for (int q = 0; q < kRows / 2; ++q) {
+                    for (int q = 0; q < kEven / 2; ++q) {
                         if (2 * q < nr) o[4 * q] = ehyl[q].x;
                         if (2 * q + 1 < nr) o[4 * q + 2] = ehyl[q].y;
                     }
@@ -1162,7 +1162,7 @@ w.src[j] = -1;
             if (x < nx) f[x + (size_t)m * pitch] = v;
         };
 #pragma unroll
-        for (int r = 0; r < kRows + 1; ++r) {
+        for (int r = 0; r < R + 1; ++r) {
             // the row below the warp's rows belongs to another warp, except row 0
             if (r == 0 ? (nr == 0 || y0 != 1) : r > nr) continue;
             const int m = y0 - 1 + r;
@@ -1178,7 +1178,7 @@ w.src[j] = -1;
             }
         }
 #pragma unroll
-        for (int j = 0; j < kRows; ++j) {
+        for (int j = 0; j < R; ++j) {
             if (j >= nr) continue;
             const int m = y0 + j;
 #pragma unroll
@@ -1193,12 +1193,12 @@ w.src[j] = -1;
             }
             if (ixe >= 0) {
                 const int xq = xe <= nc ? xe - 1 : xe - (nx - nc) + nc;
-                psi_o[psx_e + (size_t)m * 2 * nc + xq] = psx[kRows + j];
+                psi_o[psx_e + (size_t)m * 2 * nc + xq] = psx[kEven + j];
             }
             if (w.iye[j] >= 0) {
                 const int ye = m <= nc ? m - 1 : m - (ny - nc) + nc;
                 for (int x = 1 + lane; x <= nx - 1; x += 32)
-                    psi_o[psy_e + (size_t)ye * (nx + 1) + x] = psy[(kRows + 1 + j) * P + x];
+                    psi_o[psy_e + (size_t)ye * (nx + 1) + x] = psy[(R + 1 + j) * P + x];
             }
         }
     }
@@ -1207,8 +1207,12 @@ w.src[j] = -1;
 // ------------------------------------------------------------------- host side
 template <typename Real>
 using ResidentFn = void (*)(const SolveDesc<Real>*, int, int, int*);
-// The compiled kernel of a number of inner passes and a mode (null: none).
+// Rows per warp and most warps of a block.
+struct ResidentShape {
+    int share, warps;
+};
+// The compiled kernel of a number of inner passes, a mode and a shape (null: none).
 template <typename Real>
-ResidentFn<Real> resident_kernel_for(int passes, int mode);
+ResidentFn<Real> resident_kernel_for(int passes, int mode, ResidentShape shape);
 
 }  // namespace tomo

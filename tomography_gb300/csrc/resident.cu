@@ -4,6 +4,9 @@
 
 namespace tomo {
 
+// The shapes in the order of their speed: the first that holds a batch takes it.
+static constexpr ResidentShape kShapes[] = {{2, 12}, {2, 16}, {4, 12}, {4, 8}};
+
 template <typename Real>
 bool resident_plan(const ProblemClass& pc, const SolveLayout& lay, int blocks, ResidentPlan& p) {
     const tomo_spec& s = pc.spec;
@@ -21,8 +24,10 @@ bool resident_plan(const ProblemClass& pc, const SolveLayout& lay, int blocks, R
     if (right > pc.nx - std::max(pc.nc, 1)) return false;   // the x-CPML and PEC columns belong to the edge pass
     p.blocks = blocks;
     p.passes = (right - kEdge + width - 1) / width;
-    if (!resident_kernel_for<Real>(p.passes, advance_mode(s))) return false;
-    if (rows > kRows * resident_warps(p.passes) * blocks) return false;
+    bool holds = false;
+    for (const ResidentShape& q : kShapes)
+        holds |= rows <= q.share * q.warps * blocks && resident_kernel_for<Real>(p.passes, advance_mode(s), q) != nullptr;
+    if (!holds) return false;
     // staging levels in the memory of the second field copies
     p.levels = kResidentSteps;
     if (pc.nfreq > 0)
@@ -33,23 +38,29 @@ bool resident_plan(const ProblemClass& pc, const SolveLayout& lay, int blocks, R
 // Cuts rows 1 .. ny-1 into slabs of about equal cost: the least cost of the
 // dearest slab, by bisection over a greedy cut.  box: the candidate's materials.
 template <typename Real>
-static bool cut_slabs(const ProblemClass& pc, const ResidentPlan& p, const int* box, std::vector<double>& cost, int* ys,
+static bool cut_slabs(const ProblemClass& pc, const ResidentPlan& p, const ResidentShape& shape, const int* box, std::vector<double>& cost, int* ys,
                       double& dearest) {
-    const int most = kRows * resident_warps(p.passes), width = 32 * Quad<Real>::N;
-    // cost of a row, from the passes' measured times: a plain pass 0.14, one with
-    // materials or y-CPML 0.42, the rest of a row 0.6
+    const int most = shape.share * shape.warps, width = 32 * Quad<Real>::N;
+    // Cost of a row in microseconds, fitted to the step times of 200^2, 333 x 251 and 400^2
+    // grids cut in 8 to 30 ways each.  FP32 rows with materials cost up to 1.6 plain ones
+    // (400^2: 2.98 us a step, against 3.6 with equal rows), y-CPML rows 1.8.  In FP64 the
+    // arithmetic of the y-CPML rows and the staging of a face row count for more (200^2:
+    // 14.1 us a step, against 21.2 cut with the FP32 weights).
+    constexpr bool kWide = sizeof(Real) == 8;
     int mats = 0;
     for (int c = 0; c < p.passes; ++c)
         mats += box[0] < kEdge + (c + 1) * width && box[1] >= kEdge + c * width;
+    const double plain = (kWide ? 0.27 : 0.022) * p.passes, strip = (kWide ? 2.0 : 1.8) * plain;
+    const double mat = plain * (1.0 + (kWide ? 0.25 : 0.6) * mats / p.passes), face = kWide ? 6 * plain : 0;
+    const int face0 = pc.nfreq > 0 ? pc.spec.nf2ff_d : -1, face1 = pc.nfreq > 0 ? pc.ny - pc.spec.nf2ff_d - 1 : -1;
     cost.assign(pc.ny, 0.0);
     double total = 0;
     for (int m = 1; m < pc.ny; ++m) {
-        const bool strip = m <= pc.nc || m >= pc.ny - pc.nc, mat = m >= box[2] && m <= box[3];
-        cost[m] = strip ? 0.8 + 0.42 * p.passes : 0.6 + 0.14 * p.passes + (mat ? 0.28 * mats : 0.0);
+        cost[m] = m <= pc.nc || m >= pc.ny - pc.nc ? strip : m >= box[2] && m <= box[3] ? mat : plain;
+        if (m == face0 || m == face1) cost[m] += face;
         total += cost[m];
     }
     // a slab does not end at a horizontal NTFF face: its sample takes Ez of the row above
-    const int face0 = pc.nfreq > 0 ? pc.spec.nf2ff_d : -1, face1 = pc.nfreq > 0 ? pc.ny - pc.spec.nf2ff_d - 1 : -1;
     auto cut = [&](double limit) {
         int m = 1;
         for (int b = 0; b < p.blocks; ++b) {
@@ -84,32 +95,45 @@ static bool cut_slabs(const ProblemClass& pc, const ResidentPlan& p, const int* 
     return true;
 }
 
+// A batch on one shape; false: it does not fit.
 template <typename Real>
-void resident_batch(const ProblemClass& pc, const ResidentPlan& p, const Unpacked& u, ResidentBatch& b) {
+static bool batch_on(const ProblemClass& pc, const ResidentPlan& p, const ResidentShape& shape, const Unpacked& u,
+                     ResidentBatch& b) {
     const bool ref = pc.spec.mode != TOMO_MODE_BREAST;
     const int nb = p.blocks + 1, d = pc.nfreq > 0 ? pc.spec.nf2ff_d : -1, none[4] = {1, 0, 1, 0};
     const size_t n = u.ncand + pc.extra;
-    b.fits = false;
+    if (pc.ny - 1 > shape.share * shape.warps * p.blocks) return false;
+    b.shape = shape;
     b.warps = 0;
     b.smem = 0;
     b.cost = 0;
-    b.ys.resize(n * nb);
     std::vector<double> cost;
     for (size_t c = 0; c < n; ++c) {
         const int* m = c < u.ncand ? &u.mbox[4 * c] : none;
         int* ys = &b.ys[c * nb];
         if (c > 0 && c < u.ncand && std::equal(m, m + 4, m - 4)) std::copy(ys - nb, ys, ys);
-        else if (!cut_slabs<Real>(pc, p, m, cost, ys, b.cost)) return;
+        else if (!cut_slabs<Real>(pc, p, shape, m, cost, ys, b.cost)) return false;
         int tall = 0;
         for (int k = 0; k < p.blocks; ++k) tall = std::max(tall, ys[k + 1] - ys[k]);
-        b.warps = std::max(b.warps, (tall + kRows - 1) / kRows);
+        b.warps = std::max(b.warps, (tall + shape.share - 1) / shape.share);
         for (int k = 0; k < p.blocks; ++k)
-            b.smem = std::max(b.smem, resident_layout<Real>(pc.nx, pc.ny, pc.nc, pc.nmat, ref, p.passes, ys[k], ys[k + 1],
-                                                            tall, m[0], m[1], m[2], m[3], d)
+            b.smem = std::max(b.smem, resident_layout<Real>(pc.nx, pc.ny, pc.nc, pc.nmat, ref, p.passes, shape.share, ys[k],
+                                                            ys[k + 1], tall, m[0], m[1], m[2], m[3], d)
                                           .total);
     }
     b.smem = (b.smem + 4095) / 4096 * 4096;   // one captured launch serves batches of about the same boxes
-    b.fits = b.smem <= kSmemPerBlock;
+    return b.smem <= kSmemPerBlock;
+}
+
+template <typename Real>
+void resident_batch(const ProblemClass& pc, const ResidentPlan& p, const Unpacked& u, ResidentBatch& b) {
+    b.fits = false;
+    b.ys.resize((u.ncand + pc.extra) * (p.blocks + 1));
+    for (const ResidentShape& q : kShapes) {
+        if (!resident_kernel_for<Real>(p.passes, advance_mode(pc.spec), q)) continue;
+        b.fits = batch_on<Real>(pc, p, q, u, b);
+        if (b.fits) return;
+    }
 }
 
 template <typename Real>
@@ -153,7 +177,7 @@ static cudaLaunchConfig_t cluster_config(const ResidentPlan& p, const ResidentBa
 
 template <typename Real>
 int resident_clusters(const ResidentPlan& p, const ResidentBatch& b, int mode, int* clusters) {
-    ResidentFn<Real> fn = resident_kernel_for<Real>(p.passes, mode);
+    ResidentFn<Real> fn = resident_kernel_for<Real>(p.passes, mode, b.shape);
     if (!fn) return fail(TOMO_EINVAL, "no resident kernel for this grid");
     CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemPerBlock));
     CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
@@ -169,16 +193,15 @@ int resident_choice(const ProblemClass& pc, const SolveLayout& lay, const Unpack
                     ResidentBatch& b) {
     int best = -1;
     double least = 0;
-    for (int blocks : {16, 8, 4}) {
+    for (int blocks : kClusterSizes) {
         ResidentPlan q;
         if (!resident_plan<Real>(pc, lay, blocks, q)) continue;
         ResidentBatch c;
         resident_batch<Real>(pc, q, u, c);
         int clusters = 0;
         if (!c.fits || resident_clusters<Real>(q, c, advance_mode(pc.spec), &clusters)) continue;
-        // rounds of clusters, each about 1 us a step and 0.06 us per unit of the dearest slab
-        const int nsolves = (int)u.ncand * pc.n_exc;
-        const double t = ((nsolves + clusters - 1) / clusters) * (1.0 + 0.06 * c.cost);
+        if (clusters < 1) continue;
+        const double t = resident_estimate(c, (int)u.ncand * pc.n_exc, clusters);
         if (best < 0 || t < least) {
             best = blocks;
             least = t;
@@ -192,7 +215,7 @@ int resident_choice(const ProblemClass& pc, const SolveLayout& lay, const Unpack
 template <typename Real>
 int launch_resident(const ResidentPlan& p, const ResidentBatch& b, int mode, int clusters, const SolveDesc<Real>* descs,
                     int nsolves, int nsteps, int* error, cudaStream_t st) {
-    ResidentFn<Real> fn = resident_kernel_for<Real>(p.passes, mode);
+    ResidentFn<Real> fn = resident_kernel_for<Real>(p.passes, mode, b.shape);
     cudaLaunchAttribute attr;
     cudaLaunchConfig_t c = cluster_config(p, b, std::min(clusters, nsolves), st, &attr);
     CUDA_TRY(cudaLaunchKernelEx(&c, fn, descs, nsolves, nsteps, error));
