@@ -751,14 +751,26 @@ __global__ void __launch_bounds__(32 * W, 1)
                 }
             }
         }
-        for (int r = warp; r < brows; r += nwarp) {
-            const int y = L.br0 + r;
-            for (int i = lane; i < bw; i += 32) {
-                const int x = L.bx0 + i;
-                // the box's columns may reach past the inner columns by up to three: those stay vacuum
-                jp_s[r * bw + i] = x < right && n0 > 0 ? D.jp[0][x + (size_t)y * pitch] : Real(0);
-                mats_s[r * bw + i] = x < right ? D.mat[x + (size_t)y * D.mpitch] : 0;
-            }
+        // the box by Quads (its columns start on a multiple of 4, rows are padded)
+#pragma unroll 4
+        for (int i = t; i < brows * (bw / N); i += nthr) {
+            const int r = i / (bw / N), q = N * (i - r * (bw / N)), x = L.bx0 + q, y = L.br0 + r;
+            Quad<Real> v = n0 > 0 ? ldq<Real>(D.jp[0] + x + (size_t)y * pitch) : Quad<Real>{};
+            uchar4 m{};
+            const uint8_t* const mg = D.mat + x + (size_t)y * D.mpitch;
+            if (N == 4) m = *reinterpret_cast<const uchar4*>(mg);
+            else { m.x = mg[0]; m.y = mg[1]; }
+            // the box's columns may reach past the inner columns by up to three: those stay vacuum
+            uint8_t mb[4] = {m.x, m.y, m.z, m.w};
+#pragma unroll
+            for (int c = 0; c < N; ++c)
+                if (x + c >= right) {
+                    v.v[c] = Real(0);
+                    mb[c] = 0;
+                }
+            stq<Real>(jp_s + r * bw + q, v);
+#pragma unroll
+            for (int c = 0; c < N; ++c) mats_s[r * bw + q + c] = mb[c];
         }
         if (L.edge_mat)
             for (int i = t; i < brows * 32; i += nthr) {
@@ -986,6 +998,7 @@ __global__ void __launch_bounds__(32 * W, 1)
                 }
             }
             if (ypml)
+#pragma unroll 4
                 for (int x = lane; x < P; x += 32) {
 #pragma unroll
                     for (int r = 0; r < R + 1; ++r) {
@@ -1147,11 +1160,10 @@ __global__ void __launch_bounds__(32 * W, 1)
             Real* const dst = D.ez[0] + (size_t)(ya + r) * pitch;
             for (int x = N * lane; x < P; x += 32 * N) stq<Real>(dst + x, ldq<Real>(fin + (r + 1) * P + x));
         }
-        for (int r = warp; r < brows; r += nwarp)
-            for (int i = lane; i < bw; i += 32) {
-                const int x = L.bx0 + i;
-                if (x < right) D.jp[0][x + (size_t)(L.br0 + r) * pitch] = jp_s[r * bw + i];
-            }
+        for (int i = t; i < brows * (bw / N); i += nthr) {
+            const int r = i / (bw / N), q = N * (i - r * (bw / N)), x = L.bx0 + q;
+            stq_until<true>(D.jp[0] + x + (size_t)(L.br0 + r) * pitch, ldq<Real>(jp_s + r * bw + q), x, right);
+        }
         if (L.edge_mat)
             for (int i = t; i < brows * 32; i += nthr) {
                 const int ln = i & 31, x = ln < 16 ? ln : nx - 31 + ln;
