@@ -74,13 +74,14 @@ __global__ void material_table_kernel(const double* __restrict__ mp, Real* __res
     out[kCs] = (Real)((-2 * dt) / den);
 }
 
-// Progress every active solve of one kind (wavefront or resident) by T steps after
-// an advance launch; counter may be null.
+// Progress the active solves of one kind (wavefront or resident) by T steps after an
+// advance launch: `count` of them from `first` on, around the end.  counter may be null.
 template <typename Real>
-__global__ void bump_kernel(SolveDesc<Real>* descs, int nsolves, int T, int* counter, int resident) {
+__global__ void bump_kernel(SolveDesc<Real>* descs, int nsolves, int T, int* counter, int resident, int first,
+                            int count) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s == 0 && counter) *counter = 0;   // work counter of the next advance launch
-    if (s >= nsolves) return;
+    if (s >= nsolves || (s - first + nsolves) % nsolves >= count) return;
     SolveDesc<Real>& D = descs[s];
     if (D.active && D.resident == resident && D.step < D.steps_total) {
         D.step += T;

@@ -427,14 +427,30 @@ struct ResidentBatch {
     std::vector<int> ys;       // [ncand (+ 1)][blocks + 1]: first row of each slab, then ny
     double cost = 0;           // of the dearest slab: about its microseconds a step past 0.9
 };
+// A second stream of a capture, with the events that fork it off and join it.
+struct SideCapture {
+    cudaStream_t stream = nullptr;
+    cudaEvent_t ready = nullptr, summed[2] = {nullptr, nullptr};
+    int create() {
+        CUDA_TRY(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+        for (cudaEvent_t* e : {&ready, &summed[0], &summed[1]}) CUDA_TRY(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+        return TOMO_OK;
+    }
+    ~SideCapture() {
+        for (cudaEvent_t e : {ready, summed[0], summed[1]})
+            if (e) cudaEventDestroy(e);
+        if (stream) cudaStreamDestroy(stream);
+    }
+};
 inline std::array<size_t, 4> launch_key(const ResidentBatch& b) {
     return {b.smem, (size_t)b.warps, (size_t)b.shape.share, (size_t)b.shape.warps};
 }
 // Blocks per cluster on offer: of the sizes with as many clusters on the GPU the largest.
 constexpr int kClusterSizes[] = {16, 12, 10, 9, 6, 5, 4};
-// About the microseconds of a time step of nsolves solves.
+// About the microseconds of a time step of nsolves solves, of which as many run at once
+// as there are clusters.
 inline double resident_estimate(const ResidentBatch& b, int nsolves, int clusters) {
-    return ((nsolves + clusters - 1) / clusters) * (0.9 + b.cost);
+    return std::max(1.0, (double)nsolves / clusters) * (0.9 + b.cost);
 }
 // false: the class does not fit the resident kernel with that many blocks.
 template <typename Real>
@@ -453,12 +469,15 @@ void make_resident(const ProblemClass& pc, const SolveLayout& lay, const Residen
 template <typename Real>
 int resident_choice(const ProblemClass& pc, const SolveLayout& lay, const Unpacked& u, ResidentPlan& p,
                     ResidentBatch& b);
-// Clusters of the batch that run at once, and one launch of nsteps steps.
+// Clusters of the batch that run at once.
 template <typename Real>
 int resident_clusters(const ResidentPlan& p, const ResidentBatch& b, int mode, int* clusters);
+// Launches count solves from first on (around the end) on as many clusters; placed (may
+// be null) is recorded for the time when all blocks have begun.
 template <typename Real>
 int launch_resident(const ResidentPlan& p, const ResidentBatch& b, int mode, int clusters, const SolveDesc<Real>* descs,
-                    int nsolves, int nsteps, int* error, cudaStream_t st);
+                    int nsolves, int first, int count, int nsteps, int* error, cudaStream_t st,
+                    cudaEvent_t placed = nullptr);
 
 // One time step of one solve on the plain path (H, E and DFT kernels; the DFT
 // kernel only when n_contour > 0).  Returns the number of kernels launched.
@@ -471,9 +490,9 @@ inline int stage_group_for(int T) { return std::max(1, kStageLevels / std::max(T
 
 template <typename Real>
 void launch_dft(const SolveDesc<Real>* descs, int nsolves, int cmax, int fmax, int T, int n0, int nlev,
-                int resident, cudaStream_t st) {
+                int resident, cudaStream_t st, DftTasks tasks = {0, 0}) {
     dft_accumulate_kernel<Real><<<dim3(nsolves * fmax, (cmax + 127) / 128), 128, 0, st>>>(descs, T, fmax, n0, nlev,
-                                                                                              resident);
+                                                                                              resident, tasks);
 }
 
 // One advance launch (T steps of every listed solve), then -- when cmax, the
@@ -491,7 +510,7 @@ int launch_advance(const Blocking& b, int mode, int blocks, size_t smem, const S
     if (dft)
         launch_dft<Real>(descs, nsolves, cmax, fmax, b.T, dft_n0, dft_nlev, 0, st);
     bump_kernel<Real><<<(nsolves + 127) / 128, 128, 0, st>>>(const_cast<SolveDesc<Real>*>(descs), nsolves, b.T,
-                                                            counter, 0);
+                                                            counter, 0, 0, nsolves);
     return dft ? 3 : 2;
 }
 
@@ -642,6 +661,7 @@ class EngineT : public EngineBase {
     int ensure_batch(int ncand);
     int build_graph(int nlaunch);
     int autotune(size_t ncand);
+    int record_resident(int clusters, SideCapture& beside);
     int pick_resident(size_t ncand, bool* fits);
     int upload_descs(size_t ncand);
     void invalidate_graph() {
@@ -666,6 +686,7 @@ class EngineT : public EngineBase {
     std::vector<ResidentPlan> plans_;              // resident plans of the class, most blocks first
     std::vector<ResidentBatch> plan_batch_;        // the current batch on each
     size_t plan_at_ = 0;                           // the one of blk_ when blk_.blocks > 0
+    int resident_launches_ = 0;                    // of the captured graph
     std::array<size_t, 4> graph_batch_{};          // what the captured launch was made for
     Blocking items_blk_{-1, -1, -1};               // blocking the uploaded work items were cut for
     DevBuf d_tune_items_;

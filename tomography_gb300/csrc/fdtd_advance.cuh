@@ -42,6 +42,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include "packed.cuh"
 #include "solve_desc.h"
 
 namespace tomo {
@@ -139,6 +140,17 @@ __device__ __forceinline__ void acc_add<double>(double& sum, double& comp, doubl
     sum = __dadd_rn(sum, term);
 }
 
+// Two sums at once.
+__device__ __forceinline__ void acc_add2(Two<float>& sum, Two<float>& comp, Two<float> term) {
+    const Two<float> y = sub2(term, comp), t = add2(sum, y);
+    comp = sub2(sub2(t, sum), y);
+    sum = t;
+}
+__device__ __forceinline__ void acc_add2(Two<double>& sum, Two<double>& comp, Two<double> term) {
+    (void)comp;
+    sum = add2(sum, term);
+}
+
 // Contour index of a cell on a face (inverse of FDTD_common.cxx:4-46).
 __device__ __forceinline__ int contour_index_yn(int nx, int ny, int d, int x) { return x - d - 1; }
 __device__ __forceinline__ int contour_index_yp(int nx, int ny, int d, int x) {
@@ -207,32 +219,52 @@ struct Vec4<double> {
 // step, stage_group = 1: the serving loop, whose solves differ in progress).
 constexpr int kStageLevels = 8;
 
+// A pass of the DFT over the launch of the resident kernel that took the solves
+// first + i, i < count, of ntotal (ntotal = 0: all listed solves, at the same step).
+struct DftTasks {
+    int first, ntotal;      // first: index of its first task; a solve comes up every ntotal tasks
+};
+
+// The resident kernel's launches use the halves of the staging buffer in turn, so that a
+// DFT pass can run beside the next launch: the half of a launch of T steps from n0.
+template <typename Real>
+__device__ __forceinline__ size_t stage_half(const SolveDesc<Real>& D, int n0, int T) {
+    return (size_t)((n0 / T) & 1) * T * 2 * D.n_contour;
+}
+
+// Bound by issue slots (the compensated sums: four operations for each of the eight sums
+// of a frequency and contour point and step): J's and M's parts are summed as packed pairs.
 template <typename Real>
 __global__ void __launch_bounds__(128) dft_accumulate_kernel(const SolveDesc<Real>* __restrict__ descs, int T,
-                                                             int fmax, int n0_group, int nlev, int resident) {
-    const SolveDesc<Real>& D = descs[blockIdx.x / fmax];
+                                                             int fmax, int n0_group, int nlev, int resident,
+                                                             DftTasks tasks) {
+    const int task = tasks.first + blockIdx.x / fmax;
+    const SolveDesc<Real>& D = descs[tasks.ntotal ? task % tasks.ntotal : task];
+    if (tasks.ntotal) n0_group = task / tasks.ntotal * T;
     const int f = blockIdx.x % fmax;
     const int c = blockIdx.y * blockDim.x + threadIdx.x;
     const int C = D.n_contour, nfreq = D.nfreq;
     if (!D.active || D.resident != resident || f >= nfreq || c >= C) return;
     const int n0 = n0_group >= 0 ? n0_group : D.step;
     const int nsteps = min(n0_group >= 0 ? nlev : T, D.steps_total - n0);
+    if (nsteps <= 0) return;
     Real* a = D.acc + ((size_t)f * C + c) * 8;
     Real j[4], mm[4];   // J: sum re, sum im, comp re, comp im; M likewise
     Vec4<Real>::load(a, j);
     Vec4<Real>::load(a + 4, mm);
-    const Real* sp = D.stage + (size_t)c * 2;
+    Two<Real> js{j[0], j[1]}, jc{j[2], j[3]}, ms{mm[0], mm[1]}, mc{mm[2], mm[3]};
+    const Real* sp = D.stage + (resident ? stage_half(D, n0, T) : 0) + (size_t)c * 2;
     const Real* pp = D.phasor + ((size_t)n0 * nfreq + f) * 4;
 #pragma unroll 4
     for (int k = 0; k < nsteps; ++k) {
         Real p[4];
         Vec4<Real>::load(pp + (size_t)k * nfreq * 4, p);
-        const Real h = sp[(size_t)k * C * 2], e = sp[(size_t)k * C * 2 + 1];
-        acc_add(j[0], j[2], Op<Real>::mul(h, p[0]));
-        acc_add(j[1], j[3], Op<Real>::mul(h, p[1]));
-        acc_add(mm[0], mm[2], Op<Real>::mul(e, p[2]));
-        acc_add(mm[1], mm[3], Op<Real>::mul(e, p[3]));
+        const Two<Real> v = *reinterpret_cast<const Two<Real>*>(sp + (size_t)k * C * 2);
+        acc_add2(js, jc, times2(dup2<Real>(v.x), Two<Real>{p[0], p[1]}));
+        acc_add2(ms, mc, times2(dup2<Real>(v.y), Two<Real>{p[2], p[3]}));
     }
+    j[0] = js.x; j[1] = js.y; j[2] = jc.x; j[3] = jc.y;
+    mm[0] = ms.x; mm[1] = ms.y; mm[2] = mc.x; mm[3] = mc.y;
     Vec4<Real>::store(a, j);
     Vec4<Real>::store(a + 4, mm);
 }

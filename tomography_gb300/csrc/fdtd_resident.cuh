@@ -682,15 +682,17 @@ enum ResidentTodo : unsigned {
     kSourceAdd = 1u << 18      // the source goes onto the finished row
 };
 
-// Advances every listed solve by up to nsteps time steps.  gridDim.x is a
-// multiple of the cluster size; cluster q takes the solves q, q + clusters, ...
+// Advances `count` of the listed solves, from `first` on and around the end, by up
+// to nsteps time steps.  gridDim.x is a multiple of the cluster size; cluster q takes
+// the solves first + q, first + q + clusters, ...
 // The fields are read from and written to copy 0 (D.resident solves do not
 // alternate copies).  The contour samples of step D.step + k go to staging
-// level k.  *error is set when a halo row did not arrive.  The sampler reads Ez
+// level k of their half of the buffer.  *error is set when a halo row did not arrive.  The sampler reads Ez
 // of the row above a horizontal NTFF face from the same block: no slab ends at one.
 template <typename Real, int PASSES, int MODE, int R, int W>
 __global__ void __launch_bounds__(32 * W, 1)
-    fdtd_resident_kernel(const SolveDesc<Real>* __restrict__ descs, int nsolves, int nsteps, int* __restrict__ error) {
+    fdtd_resident_kernel(const SolveDesc<Real>* __restrict__ descs, int nsolves, int first, int count, int nsteps,
+                         int* __restrict__ error) {
     extern __shared__ __align__(16) unsigned char smem[];
     constexpr int N = Quad<Real>::N, P = 32 * N * PASSES + 2 * kEdge;
     constexpr bool kRef = MODE == kModeRef;
@@ -703,8 +705,8 @@ __global__ void __launch_bounds__(32 * W, 1)
     const unsigned bar0 = smem_addr(smem);
     if (threadIdx.x < 4) mbar_init(bar0 + 8 * threadIdx.x);
     int sent = 0;   // rows sent to (and taken from) each neighbour before this solve
-    for (int sv = blockIdx.x / nblk; sv < nsolves; sv += nclusters) {
-        const SolveDesc<Real>& D = descs[sv];
+    for (int task = blockIdx.x / nblk; task < count; task += nclusters) {
+        const SolveDesc<Real>& D = descs[(first + task) % nsolves];
         const int nx = D.nx, ny = D.ny, nc = D.ncpml, S = D.steps_total, n0 = D.step;
         const int ns = min(nsteps, S - n0);
         if (!D.active || ns <= 0) continue;   // the same for every block of the cluster
@@ -791,7 +793,7 @@ __global__ void __launch_bounds__(32 * W, 1)
         }
         ResidentSampler<Real>* const samp = reinterpret_cast<ResidentSampler<Real>*>(smem + L.samp);
         ResidentPoint* const points_s = reinterpret_cast<ResidentPoint*>(smem + L.points);
-        if (t == 0) *samp = {D.n_contour, S, D.nrx, L.npoints, D.traces + n0, D.stage};
+        if (t == 0) *samp = {D.n_contour, S, D.nrx, L.npoints, D.traces + n0, D.stage + stage_half(D, n0, nsteps)};
         {
             // vertical faces, then the lower and the upper horizontal face; the H buffer of a
             // step holds Hx of the two face rows, then Hy of the two face columns
@@ -1218,7 +1220,7 @@ __global__ void __launch_bounds__(32 * W, 1)
 
 // ------------------------------------------------------------------- host side
 template <typename Real>
-using ResidentFn = void (*)(const SolveDesc<Real>*, int, int, int*);
+using ResidentFn = void (*)(const SolveDesc<Real>*, int, int, int, int, int*);
 // Rows per warp and most warps of a block.
 struct ResidentShape {
     int share, warps;

@@ -28,10 +28,10 @@ bool resident_plan(const ProblemClass& pc, const SolveLayout& lay, int blocks, R
     for (const ResidentShape& q : kShapes)
         holds |= rows <= q.share * q.warps * blocks && resident_kernel_for<Real>(p.passes, advance_mode(s), q) != nullptr;
     if (!holds) return false;
-    // staging levels in the memory of the second field copies
+    // staging levels in the memory of the second field copies, two halves
     p.levels = kResidentSteps;
     if (pc.nfreq > 0)
-        p.levels = (int)std::min<size_t>(kResidentSteps, (4 * lay.field_elems - kPadLeft) / (2 * (size_t)pc.C));
+        p.levels = (int)std::min<size_t>(kResidentSteps, (4 * lay.field_elems - kPadLeft) / (4 * (size_t)pc.C));
     return p.levels >= 1;
 }
 
@@ -214,11 +214,23 @@ int resident_choice(const ProblemClass& pc, const SolveLayout& lay, const Unpack
 
 template <typename Real>
 int launch_resident(const ResidentPlan& p, const ResidentBatch& b, int mode, int clusters, const SolveDesc<Real>* descs,
-                    int nsolves, int nsteps, int* error, cudaStream_t st) {
+                    int nsolves, int first, int count, int nsteps, int* error, cudaStream_t st,
+                    cudaEvent_t placed) {
     ResidentFn<Real> fn = resident_kernel_for<Real>(p.passes, mode, b.shape);
-    cudaLaunchAttribute attr;
-    cudaLaunchConfig_t c = cluster_config(p, b, std::min(clusters, nsolves), st, &attr);
-    CUDA_TRY(cudaLaunchKernelEx(&c, fn, descs, nsolves, nsteps, error));
+    cudaLaunchAttribute attr[3];
+    cudaLaunchConfig_t c = cluster_config(p, b, std::min(clusters, count), st, attr);
+    // ahead of the DFT pass that runs beside it, whose blocks would hold up whole clusters
+    attr[1].id = cudaLaunchAttributePriority;
+    int least = 0;
+    CUDA_TRY(cudaDeviceGetStreamPriorityRange(&least, &attr[1].val.priority));
+    c.numAttrs = 2;
+    if (placed) {
+        attr[2].id = cudaLaunchAttributeLaunchCompletionEvent;
+        attr[2].val.launchCompletionEvent.event = placed;
+        attr[2].val.launchCompletionEvent.flags = 0;
+        c.numAttrs = 3;
+    }
+    CUDA_TRY(cudaLaunchKernelEx(&c, fn, descs, nsolves, first, count, nsteps, error));
     return TOMO_OK;
 }
 
@@ -231,7 +243,7 @@ int launch_resident(const ResidentPlan& p, const ResidentBatch& b, int mode, int
                                        ResidentBatch&);                                                                \
     template int resident_clusters<Real>(const ResidentPlan&, const ResidentBatch&, int, int*);                        \
     template int launch_resident<Real>(const ResidentPlan&, const ResidentBatch&, int, int, const SolveDesc<Real>*,    \
-                                       int, int, int*, cudaStream_t);
+                                       int, int, int, int, int*, cudaStream_t, cudaEvent_t);
 TOMO_RESIDENT(float)
 TOMO_RESIDENT(double)
 #undef TOMO_RESIDENT

@@ -406,11 +406,11 @@ int EngineT<Real>::serve_step(int* n_active) {
         }
         SolveDesc<Real>* const d = st->descs.template as<SolveDesc<Real>>() + r.first;
         const int steps = std::min(kServeSteps, r.plan.levels);
-        TOMO_TRY(launch_resident<Real>(r.plan, r.batch, mode, r.clusters, d, r.nsolves, steps, d_counter_.as<int>() + 1,
+        TOMO_TRY(launch_resident<Real>(r.plan, r.batch, mode, r.clusters, d, r.nsolves, 0, r.nsolves, steps, d_counter_.as<int>() + 1,
                                        stream_));
         if (dft_contour(pc) > 0)
             launch_dft<Real>(d, r.nsolves, dft_contour(pc), pc.nfreq, steps, -1, steps, 1, stream_);
-        bump_kernel<Real><<<(r.nsolves + 127) / 128, 128, 0, stream_>>>(d, r.nsolves, steps, nullptr, 1);
+        bump_kernel<Real><<<(r.nsolves + 127) / 128, 128, 0, stream_>>>(d, r.nsolves, steps, nullptr, 1, 0, r.nsolves);
         r.steps_done += steps;
     }
     for (int l = 0; l < nl; ++l)
