@@ -343,7 +343,9 @@ int post_range(const ClassData<Real>& cd, size_t ncand, const SolveDesc<Real>& f
     const int nsolves = (int)ncand * pc.n_exc;
     const size_t stride = cd.lay.per_solve;
     if (pc.nang > 0 && pc.C > 0 && d_D) {
-        dim3 grd(pc.nfreq, nsolves);
+        // blocks enough for the GPU's multiprocessors, eight angles at a time each
+        const int share = std::max(1, 1216 / std::max(1, pc.nfreq * nsolves));
+        dim3 grd(pc.nfreq, nsolves, std::min((pc.nang + 7) / 8, share));
         farfield_kernel<Real><<<grd, 256, 0, st>>>(first.acc, stride, inc_acc, pc.C, pc.nfreq, cd.freqs.template as<double>(),
                                                    cd.ffgeom.template as<double>(), cd.ffang.template as<double>(),
                                                    pc.nang, s.dx, s.ff_norm, s.pw_tau,
