@@ -152,9 +152,9 @@ struct ResidentWarp {
     // the electric form below reduces to the plain one bit for bit
     alignas(16) Real hc[kRows + 1][4], ec[kRows][4];
     Real chezdx, dx, Kp, cs, wave;    // wave: source sample of this step
-    int jp, gp, psy, tab, tab2, cpml, mats;   // places in shared memory (bytes)
+    int jp, gp, psy, tab, tab2, cpml, mats, pwcol;   // places in shared memory (bytes)
     // plane wave (reference modes); pw_t and pwf_t are of this step
-    double pw_t, pw_row[kRows], pw_kx, pw_xoff, pw_dxc0, pw_inv_tau;
+    double pw_t, pw_row[kRows], pw_dxc0, pw_inv_tau;
     float pwf_t, pwf_row[kRows], pwf_col, pwf_xoff, pwf_reach;   // the same in units of tau, for an estimate
 };
 
@@ -187,7 +187,7 @@ struct ResidentLayout {
     int npoints;             // NTFF contour points of the slab
     int hstep;               // elements of the face H of one step: two rows, two columns
     int psi_lo, psi_hi;      // warps of the slab with y-CPML rows: [0, psi_lo) and [psi_hi, warps)
-    size_t jp, gp, ejp, psy, psx, prof, cpml, tab, tab2, hf, rx, warps, samp, points, mats, emats, total;
+    size_t jp, gp, pwcol, ejp, psy, psx, prof, cpml, tab, tab2, hf, rx, warps, samp, points, mats, emats, total;
 };
 
 // share: rows per warp; [ya, yb): the slab; maxrow: the tallest slab of the cluster.
@@ -236,6 +236,7 @@ __host__ __device__ inline ResidentLayout resident_layout(int nx, int ny, int nc
     const size_t cells = brows * bw > 0 ? (size_t)brows * bw : 4;   // never empty: lanes outside read a cell too
     L.jp = take(sizeof(Real) * cells);
     L.gp = take(ref ? sizeof(Real) * (size_t)brows * bw : 0);
+    L.pwcol = take(ref ? sizeof(double) * (size_t)bw : 0);
     L.ejp = take(L.edge_mat ? sizeof(Real) * (size_t)brows * 32 : 0);
     L.psy = take(sizeof(Real) * (size_t)npsi * (2 * share + 1) * L.pitch);
     L.psx = take(nc > 0 ? sizeof(Real) * (size_t)warps * 2 * resident_even(share) * 32 : 0);
@@ -283,10 +284,11 @@ __device__ __forceinline__ void clamp_nans(Real (&v)[N]) {
 
 // Incident front exp(-((t - b) / tau)^2) at column x of row j (0 or 1) of the
 // warp, the argument in FP64 as FDTD_GPU.cu:290 has it.  t: time of the step
-// minus the offset.
+// minus the offset.  It is bound by the FP64 units, so the part of the phase that only
+// depends on the column is kept in shared memory.
 template <typename Real>
 __device__ __forceinline__ Real plane_front(const ResidentWarp<Real>& w, double t, int j, int x) {
-    const double b = __dmul_rn(__dadd_rn(w.pw_row[j], __dmul_rn(w.pw_kx, (double)x - w.pw_xoff)), w.pw_dxc0);
+    const double b = __dmul_rn(__dadd_rn(w.pw_row[j], shared_at<double>(w.pwcol)[x - w.bx0]), w.pw_dxc0);
     const Real u = (Real)__dmul_rn(__dsub_rn(t, b), w.pw_inv_tau);
     return dev_exp<Real>(-Op<Real>::mul(u, u));
 }
@@ -774,6 +776,9 @@ __global__ void __launch_bounds__(32 * W, 1)
 #pragma unroll
             for (int c = 0; c < N; ++c) mats_s[r * bw + q + c] = mb[c];
         }
+        if (kRef)   // the columns' part of a plane wave's phase
+            for (int i = t; i < bw; i += nthr)
+                reinterpret_cast<double*>(smem + L.pwcol)[i] = __dmul_rn(D.pw_kx, (double)(L.bx0 + i) - D.pw_xoff);
         if (L.edge_mat)
             for (int i = t; i < brows * 32; i += nthr) {
                 const int r = i >> 5, ln = i & 31, x = ln < 16 ? ln : nx - 31 + ln, y = L.br0 + r;
@@ -872,6 +877,7 @@ __global__ void __launch_bounds__(32 * W, 1)
         w.Kp = D.Kp;
         w.jp = (int)L.jp;
         w.gp = (int)L.gp;
+        w.pwcol = (int)L.pwcol;
         w.tab = (int)L.tab;
         w.tab2 = (int)L.tab2;
         w.cpml = (int)L.cpml;
@@ -895,8 +901,6 @@ __global__ void __launch_bounds__(32 * W, 1)
         }
         w.plane = kRef && (D.flags & kPlaneWave) != 0;
         if (kRef) {
-            w.pw_kx = D.pw_kx;
-            w.pw_xoff = D.pw_xoff;
             w.pw_dxc0 = D.pw_dxc0;
             w.pw_inv_tau = D.pw_inv_tau;
 #pragma unroll
@@ -1022,7 +1026,11 @@ __global__ void __launch_bounds__(32 * W, 1)
 #pragma unroll
             for (int j = 0; j < R; ++j)
                 if (w.jr[j] >= 0 && j < nr)
-                    for (int i = lane; i < bw; i += 32) gp_s[w.jr[j] * bw + i] = plane_front(w, t1, j, L.bx0 + i);
+                    for (int i = lane; i < bw; i += 32) {
+                        const bool near = fabsf((float)(t1 * w.pw_inv_tau) - w.pwf_row[j] -
+                                                w.pwf_col * ((float)(L.bx0 + i) - w.pwf_xoff)) < w.pwf_reach;
+                        gp_s[w.jr[j] * bw + i] = near ? plane_front(w, t1, j, L.bx0 + i) : Real(0);
+                    }
         }
         __syncwarp();
         cluster_arrive();
