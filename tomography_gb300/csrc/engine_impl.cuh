@@ -264,6 +264,8 @@ void fill_descs(const ClassData<Real>& cd, const Unpacked& u, Real* state_base, 
         D.phasor = cd.phasor.template as<Real>();
         const int* bb = &u.bbox[cand * 4];
         D.jx0 = bb[0]; D.jx1 = bb[1]; D.jy0 = bb[2]; D.jy1 = bb[3];
+        const int* mb = &u.mbox[cand * 4];
+        D.mx0 = mb[0]; D.mx1 = mb[1]; D.my0 = mb[2]; D.my1 = mb[3];
         D.dt = s.dt;
         if (s.mode == TOMO_MODE_BREAST) {
             D.flags = kPointSource;

@@ -19,6 +19,8 @@
 //  * interior block: every level of the iteration on an interior row of a
 //    strip without special columns -- all T levels as one straight-line block,
 //    so the scheduler interleaves their independent dependency chains;
+//  * background block (imaging mode, T >= 3): an interior block whose rows and
+//    columns miss the materials, without their terms and in packed pairs;
 //  * edge block (breast mode): the same for the narrow edge strips, with the
 //    x-CPML terms computed on every lane and chosen per lane by select;
 //  * otherwise per level: the fast path (interior rows, and in breast mode the
@@ -618,6 +620,16 @@ __device__ void advance_item(const SolveDesc<Real>* __restrict__ Dp, const WorkI
         }
         cp_async_commit();
     };
+    constexpr bool kBackground = !kRef && T >= 3;
+    // Iterations whose 2T rows are all outside the material box, or every one of a strip
+    // that misses its columns: the background block below.
+    int box0 = min(D.my0, jy0), box1 = max(D.my1, jy1);   // rows of the box
+    if (D.mx0 > D.mx1) { box0 = jy0; box1 = jy1; }
+    if (jx0 > jx1) { box0 = D.my0; box1 = D.my1; }
+    const bool background = kBackground && ws.tab[0][3] == Real(0);   // no Debye current either
+    const bool meets_m = D.mx0 <= D.mx1 && xs <= D.mx1 && xs + P > D.mx0, meets_j = jx0 <= jx1 && xs <= jx1 && xs + P > jx0;
+    if ((D.mx0 > D.mx1 && jx0 > jx1) || (!meets_m && !meets_j)) { box0 = 1 << 30; box1 = -1; }
+    bool no_current = false;   // the Debye registers hold zeros
     const int rstart = sweep_r0, rmax = sweep_r1;
 #pragma unroll 1
     for (int r = rstart; r < rstart + kPrefetch; ++r) issue_row(r);
@@ -631,13 +643,30 @@ __device__ void advance_item(const SolveDesc<Real>* __restrict__ Dp, const WorkI
         {
             const int slot = r & (kRowSlots - 1);
             const Real* sp = &ws.rows[slot][0][lane * COLS];
+            if constexpr (kBackground && COLS % 2 == 0) {   // a lane's columns start on an even place of the ring
 #pragma unroll
-            for (int c = 0; c < COLS; ++c) {
-                lz[c] = sp[c];
-                lx[c] = sp[P + c];
-                ly[c] = sp[2 * P + c];
-                lj[c] = sp[3 * P + c];
-                lm |= (uint32_t)ws.mats[slot][moff + lane * COLS + c] << (8 * c);
+                for (int c = 0; c < COLS; c += 2) {
+                    const Two<Real> vz = *reinterpret_cast<const Two<Real>*>(sp + c);
+                    const Two<Real> vx = *reinterpret_cast<const Two<Real>*>(sp + P + c);
+                    const Two<Real> vy = *reinterpret_cast<const Two<Real>*>(sp + 2 * P + c);
+                    const Two<Real> vj = *reinterpret_cast<const Two<Real>*>(sp + 3 * P + c);
+                    lz[c] = vz.x; lz[c + 1] = vz.y; lx[c] = vx.x; lx[c + 1] = vx.y;
+                    ly[c] = vy.x; ly[c + 1] = vy.y; lj[c] = vj.x; lj[c + 1] = vj.y;
+                }
+            } else {
+#pragma unroll
+                for (int c = 0; c < COLS; ++c) {
+                    lz[c] = sp[c];
+                    lx[c] = sp[P + c];
+                    ly[c] = sp[2 * P + c];
+                    lj[c] = sp[3 * P + c];
+                }
+            }
+            if constexpr (kBackground && COLS == 2 && T % 2 == 0) {   // the window starts on an even column
+                lm = *reinterpret_cast<const uint16_t*>(&ws.mats[slot][moff + lane * COLS]);
+            } else {
+#pragma unroll
+                for (int c = 0; c < COLS; ++c) lm |= (uint32_t)ws.mats[slot][moff + lane * COLS + c] << (8 * c);
             }
         }
 
@@ -649,7 +678,113 @@ __device__ void advance_item(const SolveDesc<Real>* __restrict__ Dp, const WorkI
         // the same for the narrow edge strips (breast mode): every level on the edge
         // path, off the y-CPML rows and inside the vertical NTFF faces' row range
         const bool edge_rows = kEdgePath && wspecial && straight;
-        if (interior) {
+        const bool plain_rows = interior && background && (r < box0 || r - 2 * T + 1 > box1);
+        if (!plain_rows) no_current = false;
+        if (plain_rows) {
+            // ---- background rows: no materials, no Debye current, the coefficients in
+            // registers and pairs of columns in packed operations.  Most of a large grid is
+            // background, and the sweep is bound by issue slots: 2048^2, T = 4 of two
+            // columns 41.3 -> 38.5 ms for 480 steps of four solves.  With two levels the
+            // rest of an iteration outweighs it (600^2: 44.2 -> 44.9 ms): not compiled there.
+            const Real Ca0 = ws.tab[0][0], Cb0 = ws.tab[0][1];
+            const Two<Real> chez2 = dup2<Real>(chez), mchez2 = dup2<Real>(-chez), ca2 = dup2<Real>(Ca0), cb2 = dup2<Real>(Cb0);
+            if (!no_current) {
+#pragma unroll
+                for (int k = 0; k < T; ++k)
+#pragma unroll
+                    for (int c = 0; c < COLS; ++c) {
+                        pj[k][c] = Real(0);
+                        hj[k][c] = Real(0);
+                    }
+                no_current = true;
+            }
+#pragma unroll
+            for (int k = T - 1; k >= 0; --k) {
+                const int m = r - 2 * k - 1;
+                Real iz[COLS], ix[COLS], iy[COLS];
+                const uint32_t im = (k == 0) ? lm : hmat[k];
+#pragma unroll
+                for (int c = 0; c < COLS; ++c) {
+                    if (k == 0) { iz[c] = lz[c]; ix[c] = lx[c]; iy[c] = ly[c]; }
+                    else { iz[c] = hz[k][c]; ix[c] = hxr[k][c]; iy[c] = hyr[k][c]; }
+                }
+                Real oz[COLS], ox[COLS], oy[COLS];
+                const Real ezR_last = __shfl_down_sync(0xffffffffu, pz[k][0], 1);
+                if constexpr (COLS % 2 == 0) {
+#pragma unroll
+                    for (int c = 0; c < COLS; c += 2) {
+                        const Two<Real> e{pz[k][c], pz[k][c + 1]};
+                        const Two<Real> d{O::sub(e.y, e.x), O::sub(c + 2 < COLS ? pz[k][(c + 2) % COLS] : ezR_last, e.y)};
+                        const Two<Real> y = fma2(chez2, d, Two<Real>{py_[k][c], py_[k][c + 1]});
+                        const Two<Real> x = fma2(mchez2, sub2(Two<Real>{iz[c], iz[c + 1]}, e), Two<Real>{px_[k][c], px_[k][c + 1]});
+                        oy[c] = y.x; oy[c + 1] = y.y; ox[c] = x.x; ox[c + 1] = x.y;
+                    }
+                } else {
+#pragma unroll
+                    for (int c = 0; c < COLS; ++c) {
+                        oy[c] = O::fma(chez, O::sub((c + 1 < COLS) ? pz[k][(c + 1) % COLS] : ezR_last, pz[k][c]), py_[k][c]);
+                        ox[c] = O::fma(-chez, O::sub(iz[c], pz[k][c]), px_[k][c]);
+                    }
+                }
+                const Real hyL_first = __shfl_up_sync(0xffffffffu, oy[COLS - 1], 1);
+                if constexpr (COLS % 2 == 0) {
+#pragma unroll
+                    for (int c = 0; c < COLS; c += 2) {
+                        const Two<Real> dHy{O::sub(oy[c], c > 0 ? oy[c > 0 ? c - 1 : 0] : hyL_first), O::sub(oy[c + 1], oy[c])};
+                        const Two<Real> dHx = sub2(Two<Real>{ox[c], ox[c + 1]}, Two<Real>{hxn[k][c], hxn[k][c + 1]});
+                        const Two<Real> z = fma2(ca2, Two<Real>{pz[k][c], pz[k][c + 1]}, mul2(cb2, sub2(dHy, dHx)));
+                        oz[c] = z.x;
+                        oz[c + 1] = z.y;
+                    }
+                } else {
+#pragma unroll
+                    for (int c = 0; c < COLS; ++c)
+                        oz[c] = O::fma(Ca0, pz[k][c], O::mul(Cb0, O::sub(O::sub(oy[c], c > 0 ? oy[c > 0 ? c - 1 : 0] : hyL_first),
+                                                                        O::sub(ox[c], hxn[k][c]))));
+                }
+#pragma unroll
+                for (int c = 0; c < COLS; ++c) {
+                    hxn[k][c] = ox[c];
+                    ezn[k][c] = oz[c];
+                }
+                if (k + 1 < T) {
+                    hmat[k + 1] = pmat[k];
+#pragma unroll
+                    for (int c = 0; c < COLS; ++c) { hz[k + 1][c] = oz[c]; hxr[k + 1][c] = ox[c]; hyr[k + 1][c] = oy[c]; }
+                } else if (m >= y0 && m < y1) {   // owned rows only
+                    const long long rowoff = (long long)m * pitch;
+                    if constexpr (COLS == 2 && T % 2 == 0) {
+                        if (owned[0]) {
+                            store_pair(ez_d + rowoff + xcol[0], oz);
+                            store_pair(hx_d + rowoff + xcol[0], ox);
+                            store_pair(hy_d + rowoff + xcol[0], oy);
+                        }
+                    } else {
+                        bool quad = false;
+                        if constexpr (COLS == 4) {
+                            quad = owned[0] && owned[3];
+                            if (quad) {
+                                store_quad(ez_d + rowoff + xcol[0], oz);
+                                store_quad(hx_d + rowoff + xcol[0], ox);
+                                store_quad(hy_d + rowoff + xcol[0], oy);
+                            }
+                        }
+                        if (!quad) {
+#pragma unroll
+                            for (int c = 0; c < COLS; ++c)
+                                if (owned[c]) {
+                                    __stcg(ez_d + rowoff + xcol[c], oz[c]);
+                                    __stcg(hx_d + rowoff + xcol[c], ox[c]);
+                                    __stcg(hy_d + rowoff + xcol[c], oy[c]);
+                                }
+                        }
+                    }
+                }
+                pmat[k] = im;
+#pragma unroll
+                for (int c = 0; c < COLS; ++c) { pz[k][c] = iz[c]; px_[k][c] = ix[c]; py_[k][c] = iy[c]; }
+            }
+        } else if (interior) {
 #pragma unroll
             for (int k = T - 1; k >= 0; --k) {
                 const int m = r - 2 * k - 1;
