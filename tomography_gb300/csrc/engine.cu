@@ -631,7 +631,8 @@ int EngineT<Real>::pick_resident(size_t ncand, bool* fits) {
 // Autotuner: times every offered blocking (T, COLS, MINB) on the actual batch
 // -- its materials, descriptors and state -- and keeps the fastest per batch
 // size.  Every blocking computes the same bits, so the choice affects speed
-// only.  Each blocking runs one warm-up launch and then about kTuneSteps time
+// only.  The fastest is timed again with a few more and fewer row segments.
+// Each blocking runs one warm-up launch and then about kTuneSteps time
 // steps from step 0 (the descriptors are re-uploaded before each); the time
 // per step (CUDA events around the timed launches) decides.  forward() then
 // sets the state up again from scratch, so tuning leaves no trace in results.
@@ -667,12 +668,15 @@ int EngineT<Real>::autotune(size_t ncand) {
     double best = 1e300;
     Blocking bestb = cands.front();
     std::vector<WorkItem> items;
-    for (const Blocking& c : cands) {
+    std::vector<Blocking> around;
+    auto segments = [&](const Blocking& c) {
+        return choose_segments((long)nsolves * items_per_solve(pc.nx, pc.ny, pc.nc, item_face_distance(pc), c.T, c.cols),
+                               pc.ny, c, num_sms_);
+    };
+    auto time = [&](Blocking c) -> int {
         items.clear();
-        const int nseg = choose_segments(
-            (long)nsolves * items_per_solve(pc.nx, pc.ny, pc.nc, item_face_distance(pc), c.T, c.cols), pc.ny, c.T,
-            24L * num_sms_);
-        append_items(items, 0, nsolves, pc.nx, pc.ny, pc.nc, item_face_distance(pc), c.T, c.cols, nseg);
+        if (!c.nseg) c.nseg = segments(c);
+        append_items(items, 0, nsolves, pc.nx, pc.ny, pc.nc, item_face_distance(pc), c.T, c.cols, c.nseg);
         TOMO_TRY(validate_items(items, 0, pc.nx, pc.ny, pc.nc, item_face_distance(pc), c.T, c.cols));
         TOMO_TRY(d_tune_items_.ensure(sizeof(WorkItem) * items.size()));
         CUDA_TRY(cudaMemcpyAsync(d_tune_items_.p, items.data(), sizeof(WorkItem) * items.size(), cudaMemcpyHostToDevice,
@@ -701,7 +705,16 @@ int EngineT<Real>::autotune(size_t ncand) {
             best = per_step;
             bestb = c;
         }
-    }
+        return TOMO_OK;
+    };
+    for (const Blocking& c : cands) TOMO_TRY(time(c));
+    if (!std::getenv("TOMO_SEGMENTS"))   // a few more and fewer segments of the fastest
+        for (const int part : {80, 90, 115, 130}) {
+            Blocking c = bestb;
+            c.nseg = std::min(bestb.nseg * part / 100, (pc.ny + 1) / std::max(12, 6 * c.T));
+            if (c.nseg >= 1 && bestb.nseg > 1 && c.nseg != bestb.nseg) around.push_back(c);
+        }
+    for (const Blocking& c : around) TOMO_TRY(time(c));
     tuned_[key] = blk_ = bestb;
     return TOMO_OK;
 }
@@ -764,13 +777,13 @@ int EngineT<Real>::ensure_batch(int ncand) {
         return TOMO_OK;
     }
     std::vector<WorkItem> items;
-    const int nseg = choose_segments(
+    const int nseg = blk_.nseg ? blk_.nseg : choose_segments(
         (long)nsolves * items_per_solve(pc.nx, pc.ny, pc.nc, item_face_distance(pc), blk_.T, blk_.cols), pc.ny,
-        blk_.T, 24L * num_sms_);
+        blk_, num_sms_);
     append_items(items, 0, nsolves, pc.nx, pc.ny, pc.nc, item_face_distance(pc), blk_.T, blk_.cols, nseg);
     TOMO_TRY(validate_items(items, 0, pc.nx, pc.ny, pc.nc, item_face_distance(pc), blk_.T, blk_.cols));
     if (nsolves != nsolves_ || (int)items.size() != nitems_ || ncand != cur_cand_ || blk_.T != items_blk_.T ||
-        blk_.cols != items_blk_.cols) {
+        blk_.cols != items_blk_.cols || nseg != items_nseg_) {
         invalidate_graph();
         TOMO_TRY(d_items_.ensure(sizeof(WorkItem) * items.size()));
         CUDA_TRY(cudaMemcpyAsync(d_items_.p, items.data(), sizeof(WorkItem) * items.size(), cudaMemcpyHostToDevice,
@@ -780,6 +793,7 @@ int EngineT<Real>::ensure_batch(int ncand) {
     nitems_ = (int)items.size();
     cur_cand_ = ncand;
     items_blk_ = blk_;
+    items_nseg_ = nseg;
     return TOMO_OK;
 }
 

@@ -115,8 +115,9 @@ int unpack_args(const ProblemClass& pc, const double* args, size_t ncand, size_t
 // that many blocks per solve.
 struct Blocking {
     int T = 1, cols = 1, minb = 2, blocks = 0;
+    int nseg = 0;   // row segments per strip (0: by choose_segments)
     bool operator==(const Blocking& o) const {
-        return T == o.T && cols == o.cols && minb == o.minb && blocks == o.blocks;
+        return T == o.T && cols == o.cols && minb == o.minb && blocks == o.blocks && nseg == o.nseg;
     }
     bool operator!=(const Blocking& o) const { return !(*this == o); }
 };
@@ -591,11 +592,14 @@ inline int items_per_solve(int nx, int ny, int ncpml, int d, int T, int cols) {
 }
 
 // Row segments per strip: 1 while a batch's strips fill the GPU, else enough
-// to reach about min_items items, keeping segments at least 6T and 12 rows
-// tall (each segment recomputes 2T halo rows; a sweep of one 4-solve call of
-// 401 rows ran fastest at about 32 segments per strip, 12-13 rows each).
-// TOMO_SEGMENTS fixes the count.
-inline int choose_segments(long strips, int ny, int T, long min_items) {
+// for one and a half items per resident warp, keeping segments at least 6T and
+// 12 rows tall.  Each segment recomputes 4T rows and fewer items than that leave
+// warps idle at the end: 2048^2 and 600^2 ran fastest at 1.3 to 1.7 items a warp
+// (two levels 24.9 and 21.8 ms, against 25.9 and 22.7 at two items; four levels of
+// 600^2 22.6 against 26.8 at three).  TOMO_SEGMENTS fixes the count.
+inline int choose_segments(long strips, int ny, const Blocking& b, int num_sms) {
+    const int T = b.T;
+    const long min_items = 6L * std::max(b.minb, 1) * num_sms;
     if (const char* e = std::getenv("TOMO_SEGMENTS")) return std::max(1, std::atoi(e));
     if (strips <= 0 || strips >= min_items) return 1;
     const int max_seg = std::max(1, (ny + 1) / std::max(12, 6 * T));
@@ -693,6 +697,7 @@ class EngineT : public EngineBase {
     int resident_launches_ = 0;                    // of the captured graph
     std::array<size_t, 4> graph_batch_{};          // what the captured launch was made for
     Blocking items_blk_{-1, -1, -1};               // blocking the uploaded work items were cut for
+    int items_nseg_ = 0;
     DevBuf d_tune_items_;
     uint64_t budget_ = (uint64_t)150 << 30;
     tomo_stats stats_{};

@@ -362,7 +362,7 @@ int EngineT<Real>::serve_step(int* n_active) {
                                                        st->blk.cols);
             nymax = std::max(nymax, pc.ny);
         }
-        const int nseg = choose_segments(strips, nymax, st->blk.T, 24L * num_sms_);
+        const int nseg = choose_segments(strips, nymax, st->blk, num_sms_);
         st->cmax = 0;
         st->fmax = 1;
         for (auto& kv : st->reqs) {
