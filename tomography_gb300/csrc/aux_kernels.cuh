@@ -198,27 +198,31 @@ __global__ void __launch_bounds__(256) farfield_kernel(const Real* __restrict__ 
 // chunk has a block of its own: the result does not depend on the batch.
 //
 // FP64 sums were bound by the FP64 units (two lanes a clock and SM, five
-// operations a sample: 596 us for 49 M samples, 5% of HBM; now 87 us, bound by
-// some 26 FP32 operations a sample).  FP32 traces are
-// summed in FP32 without their rounding errors instead: the difference, its
-// square and every addition are split into a value and its exact error (Knuth's
-// two-sum, an fma for the product), the errors are added up beside the values,
-// and a chunk's sums join in FP64.  A term keeps about 47 bits, whose rounding
-// averages out below an FP64 sum's own.  A chunk whose sum is outside [2^-70, 2^100] -- where products
-// would lose bits to underflow or overflow -- or not finite is done in FP64.
+// operations a sample: 596 us for 49 M samples, 5% of HBM; now 113 us, bound by
+// some 40 FP32 operations a sample).  FP32 traces are summed in FP32 without
+// their rounding errors instead: the difference, its square and every addition
+// are split into a value and its exact error (Knuth's two-sum, an fma for a
+// product), the errors and their errors are added up beside the values, and a
+// chunk's sums join in FP64.  Against exact sums of 1000 to 240000 samples the
+// relative error is 0.8e-16 to 1.7e-16 rms, the FP64 sums' 1.1e-16 to 1.9e-16.
+// (Without the errors' errors: 1.9e-16 to 2.5e-16, in 87 us.)  A chunk whose sum
+// is outside [2^-70, 2^100] -- where products would lose bits to underflow or
+// overflow -- or not finite is done in FP64.
 constexpr int kMisfitChunk = 8192;
 inline int misfit_chunks(size_t n_per_solve) { return (int)((n_per_solve + kMisfitChunk - 1) / kMisfitChunk); }
 
 // A sum, its error and that error's error, two columns of each.
 struct SplitSum {
     Two<float> sum{0.0f, 0.0f}, err{0.0f, 0.0f}, rest{0.0f, 0.0f};
-    // adds -m + e, with m the negative of a rounded product and e its error
-    __device__ __forceinline__ void take(Two<float> m, Two<float> e) {
+    // adds -m + e + low: m the negative of a rounded product, e its error, low what e lost
+    __device__ __forceinline__ void take(Two<float> m, Two<float> e, Two<float> low) {
         const Two<float> x = sub2(sum, m), bv = sub2(sum, x), av = add2(x, bv);
         const Two<float> y = add2(sub2(sum, av), sub2(bv, m));
         sum = x;
-        const Two<float> f = add2(y, e), z = add2(err, f), fv = sub2(z, err), ev = sub2(z, fv);
-        rest = add2(rest, add2(sub2(err, ev), sub2(f, fv)));
+        const Two<float> f = add2(y, e), ee = sub2(f, y), ye = sub2(f, ee);
+        low = add2(low, add2(sub2(y, ye), sub2(e, ee)));
+        const Two<float> z = add2(err, f), fv = sub2(z, err), ev = sub2(z, fv);
+        rest = add2(rest, add2(low, add2(sub2(err, ev), sub2(f, fv))));
         err = z;
     }
     // adds (a - b)^2
@@ -226,11 +230,14 @@ struct SplitSum {
         const Two<float> d = sub2(a, b), bv = sub2(a, d), av = add2(d, bv);
         const Two<float> lo = add2(sub2(a, av), sub2(bv, b));
         const Two<float> m{__fmul_rn(-d.x, d.x), __fmul_rn(-d.y, d.y)};
-        take(m, fma2(add2(d, d), lo, fma2(lo, lo, fma2(d, d, m))));
+        // d^2 - m and 2 d lo with its error, their sum with its error, lo^2
+        const Two<float> q = fma2(d, d, m), d2 = add2(d, d), g{__fmul_rn(d2.x, lo.x), __fmul_rn(d2.y, lo.y)};
+        const Two<float> gl = fma2(d2, lo, Two<float>{-g.x, -g.y}), u = add2(q, g), gv = sub2(u, q), qv = sub2(u, gv);
+        take(m, u, fma2(lo, lo, add2(gl, add2(sub2(q, qv), sub2(g, gv)))));
     }
     __device__ __forceinline__ void square(Two<float> a) {
         const Two<float> m{__fmul_rn(-a.x, a.x), __fmul_rn(-a.y, a.y)};
-        take(m, fma2(a, a, m));
+        take(m, fma2(a, a, m), Two<float>{0.0f, 0.0f});
     }
     // The block's sum in FP64 (thread 0): lanes, then the eight warps, in three parts.
     // (In two, the few last additions of the errors would round at 2^-49 of the sum.)
