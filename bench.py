@@ -324,8 +324,10 @@ def run_ours(args) -> None:
                 "frac": achieved / peaks["hbm_gbs"], "peak_source": peaks["source"],
                 "traffic": (tr * cells_per_launch) if tr is not None else None,
                 "algorithmic_bytes_per_launch": BYTES_PER_CELL_UPDATE * cells_per_launch,
-                "kernel": "fdtd_advance_kernel<float,%d,%d> (min %d blocks/SM)" % (
-                    st["steps_per_launch"], st["cols_per_lane"], st.get("min_blocks_per_sm", 2))}
+                "kernel": ("fdtd_resident_kernel<float>, up to %d steps a launch" % st["steps_per_launch"]
+                           if st.get("min_blocks_per_sm", 2) == 1 else
+                           "fdtd_advance_kernel<float,%d,%d> (min %d blocks/SM)" % (
+                               st["steps_per_launch"], st["cols_per_lane"], st.get("min_blocks_per_sm", 2)))}
     gcells = st["cell_updates"] * world * args.steps / tot_dev / 1e9
 
     extra = {}

@@ -538,7 +538,7 @@ int EngineT<Real>::upload_descs(size_t ncand) {
     if (pc.extra)
         h_descs_[nsolves - 1] =
             incident_desc<Real>(cd_, d_state_.as<Real>() + (size_t)(nsolves - 1) * cd_.lay.per_solve);
-    if (blk_.blocks > 0) 
+    if (blk_.blocks > 0)
         make_resident<Real>(pc, cd_.lay, plans_[plan_at_], plan_batch_[plan_at_], up_, h_descs_.data(), nsolves);
     else if (!pc.spec.plain)   // the time-loop graph runs one DFT pass per group of launches
         for (SolveDesc<Real>& D : h_descs_) D.stage_group = stage_group_for(blk_.T);

@@ -7,7 +7,7 @@
 // by many time steps without touching HBM, and writes it back.
 //
 // Layout.  The rows 1 .. ny-1 of the Ez grid are cut into one slab per block
-// (SolveDesc::ys), a slab into groups of four rows, one group per warp:
+// (SolveDesc::ys), a slab into groups of two (four) rows, one group per warp:
 //  * Ez of a slab lives in shared memory, two copies (time n and n+1), with one
 //    halo row below and above that the neighbouring blocks write through
 //    distributed shared memory;
@@ -24,8 +24,22 @@
 // ones, so every cell gets the bits of the other paths.
 //
 // A step ends with one block barrier; blocks wait for each other's halo rows
-// only.  Then all threads of a block sample the step together: the receivers to
-// the traces and the NTFF contour to the staging buffer.
+// only.  Then the threads of a block sample the step, the warps with the fewest
+// rows first: the receivers to the traces and the NTFF contour to the staging buffer.
+//
+// What bounds it.  Latency and issue of few warps: a block with materials issues on
+// 30% of its slots and uses the shared memory pipe at 47%, and a step cannot be
+// shorter than the slowest warp's passes (400^2, cluster of 16: about 500 cycles
+// of halo wait, 900 of edge pass, 500 to 1200 a pass, 400 of sampling).  So a
+// warp holds as few rows as the registers allow: with two rows, 16 warps of 128
+// registers (12 of 168 in FP64 and where 24 rows a block are enough) a step takes
+//   400^2  2.98 us, against 3.60 with four rows and 8 warps of 255 registers,
+//   200^2  1.69 us, against 2.53;   333 x 251  2.00 us, against 2.91,
+//   FP64 200^2  14.1 us, against 25.0 (bound by the FP64 units, two lanes a clock).
+// Three rows (12 warps) spill and run at 3.64 us on 400^2.  Ez of a warp's own
+// rows kept in registers too: 4.19 us, the four-row passes lose the room to load ahead.
+// Four rows stay where two would not hold the grid: 512 columns, tall narrow grids.
+// The wavefront kernel took 14.3 ms for a 200^2 forward of 1000 steps, this one 2.2.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -91,9 +105,9 @@ __device__ __forceinline__ unsigned remote_addr(unsigned local, unsigned rank) {
 }
 // A halo row travels as one bulk copy between the shared memories: it counts its
 // bytes on an mbarrier of the receiving block, whose reader waits for them.
-// Neighbours need no other synchronisation.  (A cluster barrier per step costs a
-// fence for the block's global stores and empties the first-level cache; a row of
-// 16-byte st.async, one count each, arrived 2.7 us after it was sent.)
+// Neighbours need no other synchronisation.  (A cluster barrier per step waits for the
+// slowest block of all and costs a fence for the block's global stores: 5.6 us a step on
+// 400^2 where this took 4.1.  Stores of 16 bytes, one count each, took 4.3.)
 __device__ __forceinline__ void mbar_init(unsigned bar) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
