@@ -5,10 +5,11 @@
 //         triples and ellipse geometry (FDTD_GPU.cu:657-693 / FDTD_CPU.cxx:682-698)
 //   H2D : one packed upload
 //   GPU : material maps + FP64 coefficient tables, zero state, a CUDA graph of
-//         ceil(steps/T) advance launches (each followed by the running DFT of
-//         the NTFF contour and a progress bump), far field, misfit; the
-//         blocking of the advance kernel is autotuned on the first batch of
-//         each size
+//         launches of the resident kernel where the grid fits a thread-block
+//         cluster (parts of the time loop, the DFT of a launch beside the next),
+//         else ceil(steps/T) advance launches (each followed by the running DFT
+//         of the NTFF contour and a progress bump), far field, misfit; the
+//         cluster size or the blocking is tuned on the first batch of each size
 //   D2H : fitness (plus optional traces / far field)
 // Device buffers persist across calls (the reference allocates and frees ~30
 // buffers inside every call, FDTD_GPU.cu:858-1106).
