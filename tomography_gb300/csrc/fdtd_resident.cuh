@@ -43,6 +43,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include "cluster.cuh"
 #include "fdtd_advance.cuh"
 #include "packed.cuh"
 #include "solve_desc.h"
@@ -85,72 +86,6 @@ __device__ __forceinline__ Two<Real> half_of(const Quad<Real>& q, int i) {
     return {q.v[2 * i], q.v[2 * i + 1]};
 }
 
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-__device__ __forceinline__ unsigned cluster_rank() {
-    unsigned r;
-    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ unsigned cluster_blocks() {
-    unsigned r;
-    asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ unsigned remote_addr(unsigned local, unsigned rank) {
-    unsigned r;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local), "r"(rank));
-    return r;
-}
-// A halo row travels as one bulk copy between the shared memories: it counts its
-// bytes on an mbarrier of the receiving block, whose reader waits for them.
-// Neighbours need no other synchronisation.  (A cluster barrier per step waits for the
-// slowest block of all and costs a fence for the block's global stores: 5.6 us a step on
-// 400^2 where this took 4.1.  Stores of 16 bytes, one count each, took 4.3.)
-__device__ __forceinline__ void mbar_init(unsigned bar) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-__device__ __forceinline__ void mbar_arm(unsigned bar, unsigned bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_try(unsigned bar, unsigned parity) {
-    unsigned ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-__device__ __forceinline__ void proxy_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void copy_row(unsigned dst, unsigned src, unsigned bytes, unsigned bar) {
-    asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-                 "r"(src), "r"(bytes), "r"(bar)
-                 : "memory");
-}
-// Waits for a halo row; false when it did not come within about two seconds,
-// which no correct run meets: the caller then reports it and waits no more.
-constexpr long long kHaloClocks = 4000000000ll;
-__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity) {
-    if (mbar_try(bar, parity)) return true;
-    const long long start = clock64();
-    while (clock64() - start < kHaloClocks)
-        if (mbar_try(bar, parity)) return true;
-    return false;
-}
-
-// A place in the block's dynamic shared memory.  Pointers kept in memory lose
-// their address space (and cost generic loads), so tables are kept as offsets.
-template <typename T>
-__device__ __forceinline__ T* shared_at(size_t offset) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    return reinterpret_cast<T*>(smem + offset);
-}
-
 // What a warp's longer passes need beside the fields.  It lives in shared memory
 // (one per warp): in registers it would push the fields out to local memory, and
 // with this kernel's shared memory the first-level cache is too small for that.
@@ -190,7 +125,9 @@ struct ResidentSampler {
 // Byte offsets of one block's shared memory.  The halo barriers and the Ez copies
 // come first: they are placed alike in every block of the cluster, whose
 // neighbours write into them.
-constexpr int kBarBytes = 128;   // four mbarriers, padded
+constexpr int kBarBytes = 128;   // four mbarriers, the words below, padded
+constexpr int kLostAt = 32;      // not 0: a halo row did not come, and the whole cluster gives up
+constexpr int kIssuedAt = 36;    // rows sent to the block below, and above, by the end of a solve
 
 struct ResidentLayout {
     int pitch;               // elements per Ez row
@@ -703,13 +640,14 @@ enum ResidentTodo : unsigned {
 // the solves first + q, first + q + clusters, ...
 // The fields are read from and written to copy 0 (D.resident solves do not
 // alternate copies).  The contour samples of step D.step + k go to staging
-// level k of their half of the buffer.  *error is set when a halo row did not arrive.  The sampler reads Ez
+// level k of their half of the buffer.  *error is set when a halo row did not arrive: the
+// cluster then gives up together, at the end of the solve.  The sampler reads Ez
 // of the row above a horizontal NTFF face from the same block: no slab ends at one.
 template <typename Real, int PASSES, int MODE, int R, int W>
 __global__ void __launch_bounds__(32 * W, 1)
     fdtd_resident_kernel(const SolveDesc<Real>* __restrict__ descs, int nsolves, int first, int count, int nsteps,
                          int* __restrict__ error) {
-    extern __shared__ __align__(16) unsigned char smem[];
+    unsigned char* const smem = shared_at<unsigned char>(0);
     constexpr int N = Quad<Real>::N, P = 32 * N * PASSES + 2 * kEdge;
     constexpr bool kRef = MODE == kModeRef;
     constexpr int kEven = resident_even(R);
@@ -719,7 +657,9 @@ __global__ void __launch_bounds__(32 * W, 1)
     // barriers of the row below (two, used in turn) and of the row above; they count
     // on from solve to solve
     const unsigned bar0 = smem_addr(smem);
+    volatile int* const lost = reinterpret_cast<volatile int*>(smem + kLostAt);
     if (threadIdx.x < 4) mbar_init(bar0 + 8 * threadIdx.x);
+    if (threadIdx.x == 0) *lost = 0;
     int sent = 0;   // rows sent to (and taken from) each neighbour before this solve
     for (int task = blockIdx.x / nblk; task < count; task += nclusters) {
         const SolveDesc<Real>& D = descs[(first + task) % nsolves];
@@ -1046,6 +986,7 @@ __global__ void __launch_bounds__(32 * W, 1)
                         gp_s[w.jr[j] * bw + i] = near ? plane_front(w, t1, j, L.bx0 + i) : Real(0);
                     }
         }
+        proxy_fence();   // the halo rows, zeroed here, are written by the neighbours' copies from now on
         __syncwarp();
         cluster_arrive();
         cluster_wait();
@@ -1057,7 +998,7 @@ __global__ void __launch_bounds__(32 * W, 1)
         // The warp that owns the slab's first row takes the row below from that
         // block and sends it its own; likewise the last row and the block above.
         const int src_at = has_src ? (D.src_y - ya + 1) * P + D.src_x : 0;
-        bool alive = true;
+        int until = ns;   // the step at which the warp gave up its exchange
         for (int k = 0; k < ns; ++k) {
             Real* const cur = ez_s + (k & 1) * copy;
             Real* const nxt = ez_s + (~k & 1) * copy;
@@ -1066,13 +1007,17 @@ __global__ void __launch_bounds__(32 * W, 1)
                 // neighbour is at most one message ahead
                 const int m = sent + k - 1;
                 const unsigned parity = (m >> 1) & 1, slot8 = 8 * (unsigned)(m & 1);
-                if (k > 0 && alive) {
-                    if (todo & kBelow) alive = mbar_wait(bar0 + slot8, parity);
-                    if ((todo & kAbove) && alive) alive = mbar_wait(bar0 + 16 + slot8, parity);
-                    if (!alive) *error = 1;
+                bool came = true;
+                if (k > 0 && k < until) {
+                    if (todo & kBelow) came = mbar_wait(bar0 + slot8, parity, lost);
+                    if ((todo & kAbove) && came) came = mbar_wait(bar0 + 16 + slot8, parity, lost);
                 }
-                __syncwarp();
-                if (k + 1 < ns && lane == 0) {
+                if (__any_sync(0xffffffffu, !came)) {
+                    until = k;
+                    *error = 1;
+                    if (lane < nblk) remote_store(remote_addr(bar0 + kLostAt, lane), 1);
+                }
+                if (k + 1 < ns && k < until && lane == 0) {
                     const unsigned bytes = (unsigned)(P * sizeof(Real)), next8 = 8 * (unsigned)((m + 1) & 1);
                     if (todo & kBelow) mbar_arm(bar0 + next8, bytes);
                     if (todo & kAbove) mbar_arm(bar0 + 16 + next8, bytes);
@@ -1157,7 +1102,7 @@ __global__ void __launch_bounds__(32 * W, 1)
                     }
                 }
                 // boundary rows of the slab to the neighbours' halo rows
-                if ((todo & (kBelow | kAbove)) && k + 1 < ns) {
+                if ((todo & (kBelow | kAbove)) && k + 1 < ns && k < until) {
                     proxy_fence();   // the row is written by every lane, and read by the copy
                     __syncwarp();
                     if (lane == 0) {
@@ -1176,7 +1121,14 @@ __global__ void __launch_bounds__(32 * W, 1)
             if (todo & kSample)
                 resident_sample<Real, P>(*samp, rx_s, points_s, nxt, hf_s + (k & 1) * L.hstep, k);
         }
-        sent += ns - 1;
+        // The neighbours have not answered the last row sent to them.  A block may overwrite
+        // its rows, or end, once every block of the cluster has waited for its own; the
+        // write-back hides the barrier.
+        const int issued = sent + (until < ns ? until : ns - 1);
+        if (lane == 0 && (todo & kBelow)) reinterpret_cast<int*>(smem + kIssuedAt)[0] = issued;
+        if (lane == 0 && (todo & kAbove)) reinterpret_cast<int*>(smem + kIssuedAt)[1] = issued;
+        __syncwarp();
+        cluster_arrive();
 
         // ---- write the slab back
         const Real* const fin = ez_s + (ns & 1) * copy;
@@ -1237,6 +1189,25 @@ __global__ void __launch_bounds__(32 * W, 1)
                     psi_o[psy_e + (size_t)ye * (nx + 1) + x] = psy[(R + 1 + j) * P + x];
             }
         }
+        __syncwarp();
+        cluster_wait();
+        if (*lost) {   // the same in every block
+            // rows that are still on their way: none may arrive after its receiver has ended
+            auto drain = [&](unsigned bar, unsigned theirs) {
+                for (int m = sent + until - 1, end = remote_load(theirs); m < end; ++m) {
+                    if (m >= issued && lane == 0) mbar_arm(bar + 8 * (unsigned)(m & 1), (unsigned)(P * sizeof(Real)));
+                    __syncwarp();
+                    if (!__all_sync(0xffffffffu, mbar_wait(bar + 8 * (unsigned)(m & 1), (m >> 1) & 1, nullptr))) return;
+                }
+            };
+            if (todo & kBelow) drain(bar0, remote_addr(bar0 + kIssuedAt + 4, rank - 1));
+            if (todo & kAbove) drain(bar0 + 16, remote_addr(bar0 + kIssuedAt, rank + 1));
+            __syncwarp();
+            cluster_arrive();
+            cluster_wait();
+            return;
+        }
+        sent += ns - 1;
     }
 }
 
