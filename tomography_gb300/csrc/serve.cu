@@ -61,11 +61,13 @@ struct ServeRequest {
     int* flag = nullptr;
     std::vector<double> fitness;
     int hflag = 0;
+    bool advances() const { return state == kRunning && mem; }
 };
 
 template <typename Real>
 struct ServeStateT {
     DevBuf descs, items;
+    DevBuf lost;   // error words of the resident kernel, a request's at its first slot
     std::vector<SolveDesc<Real>> hdescs;
     std::vector<char> used;
     std::map<uint64_t, std::unique_ptr<ServeRequest<Real>>> reqs;
@@ -100,6 +102,9 @@ static ServeStateT<Real>* serve_state(ServeStateT<Real>*& s, int* rc) {
     *rc = st->descs.ensure(sizeof(SolveDesc<Real>) * kServeSlots);
     if (*rc == TOMO_OK && cudaMemset(st->descs.p, 0, sizeof(SolveDesc<Real>) * kServeSlots) != cudaSuccess)
         *rc = fail(TOMO_ECUDA, "cudaMemset of serving descriptors failed");
+    if (*rc == TOMO_OK) *rc = st->lost.ensure(sizeof(int) * kServeSlots);
+    if (*rc == TOMO_OK && cudaMemset(st->lost.p, 0, sizeof(int) * kServeSlots) != cudaSuccess)
+        *rc = fail(TOMO_ECUDA, "cudaMemset of the serving error words failed");
     if (*rc) {
         delete st;
         return nullptr;
@@ -271,6 +276,7 @@ static int admit(EngineT<Real>* eng, ServeStateT<Real>* st, ServeRequest<Real>& 
         TOMO_TRY(setup_materials<Real>(cd, r.up, r.upload, r.mats, r.tabs, stream, &kernels, &h2d));
         CUDA_TRY(cudaMemsetAsync(r.state_base, 0, b_state, stream));
         CUDA_TRY(cudaMemsetAsync(r.flag, 0, sizeof(int), stream));
+        CUDA_TRY(cudaMemsetAsync(st->lost.template as<int>() + first, 0, sizeof(int), stream));
         fill_descs<Real>(cd, r.up, r.state_base, r.mats, r.tabs, &st->hdescs[first]);
         r.resident = resident && resident_choice<Real>(cd.pc, cd.lay, r.up, r.plan, r.batch) > 0;
         if (r.resident) {
@@ -356,7 +362,7 @@ int EngineT<Real>::serve_step(int* n_active) {
         int nymax = 0;
         for (auto& kv : st->reqs) {
             const ServeRequest<Real>& r = *kv.second;
-            if (r.state != kRunning || r.resident) continue;
+            if (!r.advances() || r.resident) continue;
             const ProblemClass& pc = r.cd->pc;
             strips += (long)r.nsolves * items_per_solve(pc.nx, pc.ny, pc.nc, item_face_distance(pc), st->blk.T,
                                                        st->blk.cols);
@@ -367,7 +373,7 @@ int EngineT<Real>::serve_step(int* n_active) {
         st->fmax = 1;
         for (auto& kv : st->reqs) {
             const ServeRequest<Real>& r = *kv.second;
-            if (r.state != kRunning || r.resident) continue;
+            if (!r.advances() || r.resident) continue;
             const size_t n0 = items.size();
             const ProblemClass& pc = r.cd->pc;
             append_items(items, r.first, r.nsolves, pc.nx, pc.ny, pc.nc, item_face_distance(pc), st->blk.T,
@@ -392,13 +398,14 @@ int EngineT<Real>::serve_step(int* n_active) {
     // of up to kServeSteps steps each (the kernel ends at a solve's last step).
     // The others together: as many wavefront launches as the one closest to its
     // end still needs, at most kLaunchesPerStep, so that no request runs past its
-    // last step.  The host synchronises once per serving step.
+    // last step.  The host synchronises after the launches, and once more for what they retire.
     constexpr int kServeSteps = 128, kLaunchesPerStep = 4;
     const int mode = advance_mode(cd_.pc.spec);
     int running = 0, nl = st->nitems > 0 ? kLaunchesPerStep : 0;
+    bool resident = false;
     for (auto& kv : st->reqs) {
         ServeRequest<Real>& r = *kv.second;
-        if (r.state != kRunning) continue;
+        if (!r.advances()) continue;
         const ProblemClass& pc = r.cd->pc;
         if (!r.resident) {
             nl = std::min(nl, (pc.S - r.steps_done + st->blk.T - 1) / st->blk.T);
@@ -406,8 +413,9 @@ int EngineT<Real>::serve_step(int* n_active) {
         }
         SolveDesc<Real>* const d = st->descs.template as<SolveDesc<Real>>() + r.first;
         const int steps = std::min(kServeSteps, r.plan.levels);
-        TOMO_TRY(launch_resident<Real>(r.plan, r.batch, mode, r.clusters, d, r.nsolves, 0, r.nsolves, steps, d_counter_.as<int>() + 1,
-                                       stream_));
+        TOMO_TRY(launch_resident<Real>(r.plan, r.batch, mode, r.clusters, d, r.nsolves, 0, r.nsolves, steps,
+                                       st->lost.template as<int>() + r.first, stream_));
+        resident = true;
         if (dft_contour(pc) > 0)
             launch_dft<Real>(d, r.nsolves, dft_contour(pc), pc.nfreq, steps, -1, steps, 1, stream_);
         bump_kernel<Real><<<(r.nsolves + 127) / 128, 128, 0, stream_>>>(d, r.nsolves, steps, nullptr, 1, 0, r.nsolves);
@@ -418,20 +426,30 @@ int EngineT<Real>::serve_step(int* n_active) {
                              st->items.template as<WorkItem>(), st->nitems, st->hi_slot, d_counter_.as<int>(), st->cmax,
                              st->fmax, stream_);
     CUDA_TRY(cudaGetLastError());
+    std::vector<int> lost(resident ? st->hi_slot : 0);
+    if (resident) {
+        CUDA_TRY(cudaMemcpyAsync(lost.data(), st->lost.p, sizeof(int) * lost.size(), cudaMemcpyDeviceToHost, stream_));
+        CUDA_TRY(cudaStreamSynchronize(stream_));
+    }
+    // a request whose halo row did not arrive has no result: it fails, and returns what it holds
+    bool failed = false;
     for (auto& kv : st->reqs) {
         ServeRequest<Real>& r = *kv.second;
-        if (r.state != kRunning) continue;
+        if (!r.advances() || !r.resident || !lost[r.first]) continue;
+        failed = true;
+        TOMO_TRY(retire(st, r, stream_, false));
+        r.state = kFailed;
+        r.status = TOMO_ECUDA;
+        r.up = Unpacked{};
+    }
+    for (auto& kv : st->reqs) {
+        ServeRequest<Real>& r = *kv.second;
+        if (!r.advances()) continue;
         if (!r.resident) r.steps_done += nl * st->blk.T;
         if (r.steps_done >= r.cd->pc.S) TOMO_TRY(retire(st, r, stream_, true));
         else ++running;
     }
-    int lost = 0;
-    CUDA_TRY(cudaMemcpyAsync(&lost, d_counter_.as<int>() + 1, sizeof(int), cudaMemcpyDeviceToHost, stream_));
     CUDA_TRY(cudaStreamSynchronize(stream_));
-    if (lost) {
-        CUDA_TRY(cudaMemset(d_counter_.as<int>() + 1, 0, sizeof(int)));
-        return fail(TOMO_ECUDA, "internal error: a halo row of the resident kernel did not arrive");
-    }
     for (auto& kv : st->reqs) {
         ServeRequest<Real>& r = *kv.second;
         if (r.state == kRunning && r.mem == nullptr) {
@@ -450,6 +468,7 @@ int EngineT<Real>::serve_step(int* n_active) {
     stats_.serve_queued = queued;
     stats_.serve_running_solves = solves;
     if (n_active) *n_active = running + queued;
+    if (failed) return fail(TOMO_ECUDA, "internal error: a halo row of the resident kernel did not arrive");
     return TOMO_OK;
 }
 
