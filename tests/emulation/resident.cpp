@@ -1,9 +1,11 @@
-// Runs the resident kernel's source on host threads: resident <blocks> <steps> <what>,
+// Runs the resident kernel's source on host threads:
+// resident <nx> <ny> <ncpml> <blocks> <steps> <receivers> <what>, with <what>
 //   late    copies into block 0 come 0.1 s after they were issued; two solves in turn
 //   lost    the second row sent to block 1 never comes
 //   slow    it comes after the receiver's limit
-// "late" has to give each solve's bits of a launch of its own; in the others the launch
-// has to end with its error word set.  In none may a copy touch a block that has ended.
+//   ends    nothing of the kind: the traces end in the final field
+// "late" has to give each solve's bits of a launch of its own; with "lost" and "slow" the
+// launch has to end with its error word set.  Never may a copy touch a block that has ended.
 #include "fdtd_resident.cuh"
 
 #include <cstdlib>
@@ -99,10 +101,10 @@ static int launch(std::vector<SolveDesc<Real>> descs, int blocks, std::function<
 }
 
 int main(int argc, char** argv) {
-    if (argc < 7) return 2;
+    if (argc < 8) return 2;
     const int nx = std::atoi(argv[1]), ny = std::atoi(argv[2]), nc = std::atoi(argv[3]), blocks = std::atoi(argv[4]),
-              steps = std::atoi(argv[5]), nrx = 5;
-    const std::string what = argv[6];
+              steps = std::atoi(argv[5]), nrx = std::atoi(argv[6]);
+    const std::string what = argv[7];
     int faults = 0, bad = 0;
     Solve got[2], want[2];
     std::vector<SolveDesc<Real>> both;
@@ -113,11 +115,17 @@ int main(int argc, char** argv) {
         bad += launch({want[i].d}, blocks, nullptr, &faults) != 0;
     }
     auto delay = [&](int to, int index) {
+        if (what == "ends") return 0.0;
         if (what == "late") return to == 0 ? 0.1 : 0.0;
         return to == 1 && index == 1 ? (what == "lost" ? -1.0 : 1.3) : 0.0;
     };
     const int error = launch(both, blocks, delay, &faults);
-    if (what == "late") {
+    if (what == "ends") {
+        for (int r = 0; r < nrx; ++r) {
+            const int x = got[0].rx[2 * r], y = got[0].rx[2 * r + 1];
+            bad += got[0].traces[(size_t)r * (steps + 1) + steps] != got[0].d.ez[0][x + (size_t)y * got[0].d.pitch];
+        }
+    } else if (what == "late") {
         bad += error != 0;
         for (int i = 0; i < 2; ++i) {
             bad += std::memcmp(got[i].fields.data(), want[i].fields.data(), sizeof(Real) * got[i].fields.size()) != 0;

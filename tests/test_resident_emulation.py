@@ -40,11 +40,17 @@ def _run(exe, *args):
 @pytest.mark.parametrize("blocks,steps", [(2, 2), (2, 3), (3, 4)])
 def test_late_rows(emulated, share, blocks, steps):
     """No block overwrites its rows, or ends, before its neighbour has its last one."""
-    _run(emulated[share], 64, 8 * blocks + 1, 4, blocks, steps, "late")
+    _run(emulated[share], 64, 8 * blocks + 1, 4, blocks, steps, 5, "late")
 
 
 @pytest.mark.parametrize("what", ["lost", "slow"])
 @pytest.mark.parametrize("blocks,steps", [(2, 5), (3, 6), (4, 3)])
 def test_rows_that_do_not_come(emulated, what, blocks, steps):
     """The whole cluster gives up, reports it, and no row arrives after its end."""
-    _run(emulated[2], 64, 8 * blocks + 1, 4, blocks, steps, what)
+    _run(emulated[2], 64, 8 * blocks + 1, 4, blocks, steps, 5, what)
+
+
+@pytest.mark.parametrize("share,rows", [(4, 4), (4, 6), (2, 4)])
+def test_every_receiver_is_sampled(emulated, share, rows):
+    """64 receivers on blocks of one warp, and of two."""
+    _run(emulated[share], 90, 3 * rows + 1, 0, 3, 3, 64, "ends")

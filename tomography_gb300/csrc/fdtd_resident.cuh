@@ -614,7 +614,9 @@ template <typename Real, int P>
 __device__ __forceinline__ void resident_sample(const ResidentSampler<Real>& q, const int* rx,
                                                 const ResidentPoint* points, const Real* nxt, const Real* h, int k) {
     const int t = blockDim.x - 1 - threadIdx.x;   // the last warps first: they may have no rows
-    if (t < q.nrx && rx[t] >= 0) q.traces[(size_t)t * q.S + k] = nxt[rx[t]];
+    // most often one receiver a thread at most, but a block may have one warp alone
+    for (int i = t; i < q.nrx; i += blockDim.x)
+        if (rx[i] >= 0) q.traces[(size_t)i * q.S + k] = nxt[rx[i]];
     for (int i = t; i < q.total; i += blockDim.x) {
         const ResidentPoint p = points[i];
         const Real* z = nxt + p.ez;
