@@ -1,4 +1,4 @@
-"""Failures of the resident kernel's launches, made on the host: a copy of the library is
+"""Failures of the resident kernel's launches and of its occupancy query, made on the host: a copy of the library is
 linked against CUDA calls that fail on request (tests/failing_runtime).  No launch fails or
 hangs on the GPU."""
 from __future__ import annotations
@@ -13,7 +13,7 @@ from helpers import small_breast_spec, small_params
 
 pytestmark = pytest.mark.gpu
 
-WRAPPED = ("cudaLaunchKernelExC",)
+WRAPPED = ("cudaLaunchKernelExC", "cudaOccupancyMaxActiveClusters")
 ECUDA = -5
 
 
@@ -91,3 +91,28 @@ def test_serving(failing, launch):
                 np.testing.assert_array_equal(s.poll(t, len(want[i])), want[i])
         t = s.submit(a)                              # the slots and the words are free again
         np.testing.assert_array_equal(s.wait(t, 2, 60.0), want[0])
+
+
+@pytest.mark.parametrize("error", [0, 1])
+@pytest.mark.parametrize("most", [12, 5, 0])
+def test_cluster_sizes_that_do_not_fit(failing, most, error):
+    """Where the GPU has no room for a cluster size, a smaller one or the wavefront kernel
+    serves the call, with the same bits, before and after a first choice."""
+    from tomography_gb300 import workloads as W
+
+    lib = failing.library()
+    with _solver(failing, W) as s:
+        a = _cands(W, 3, 21)
+        want = s.fitness_batch(a)
+        try:
+            lib.failing_most_blocks(most, error)
+            got = s.fitness_batch(a[:2])
+            assert (s.stats()["min_blocks_per_sm"] == 1) == (most > 0)
+            np.testing.assert_array_equal(got, want[:2])
+            np.testing.assert_array_equal(s.fitness_batch(a), want)
+            np.testing.assert_array_equal(s.wait(s.submit(a), 3, 60.0), want)
+            with _solver(failing, W) as fresh:
+                np.testing.assert_array_equal(fresh.fitness_batch(a), want)
+        finally:
+            lib.failing_most_blocks(1 << 30, 0)
+        np.testing.assert_array_equal(s.fitness_batch(a), want)

@@ -552,7 +552,8 @@ int EngineT<Real>::upload_descs(size_t ncand) {
 // Sets blk_ and plan_at_ to the resident plan of a batch, if one fits.  The plan of a
 // batch size is chosen once: of the three with the least estimated time, the fastest
 // measured (a launch of 40 steps less one of 8: the slabs' loading and storing cancels).
-// A batch that the chosen one does not hold takes the one with the least estimate.
+// A batch that the chosen one does not hold takes the one with the least estimate.  A
+// cluster size that the GPU has no room for is passed over.
 template <typename Real>
 int EngineT<Real>::pick_resident(size_t ncand, bool* fits) {
     constexpr int kShort = 8, kLong = 40;
@@ -567,8 +568,13 @@ int EngineT<Real>::pick_resident(size_t ncand, bool* fits) {
     };
     const auto known = tuned_resident_.find(key);
     if (known != tuned_resident_.end()) {
-        resident_batch<Real>(pc, plans_[known->second], up_, plan_batch_[known->second]);
-        if (plan_batch_[known->second].fits) {
+        const ResidentPlan& p = plans_[known->second];
+        ResidentBatch& b = plan_batch_[known->second];
+        resident_batch<Real>(pc, p, up_, b);
+        // the captured graph's launch has been placed before; another one is asked for
+        int clusters = graph_exec_ && graph_blk_.blocks == p.blocks && graph_batch_ == launch_key(b) ? 1 : 0;
+        if (b.fits && !clusters) TOMO_TRY(resident_clusters<Real>(p, b, mode, &clusters));
+        if (b.fits && clusters > 0) {
             use(known->second);
             return TOMO_OK;
         }
@@ -848,8 +854,10 @@ int EngineT<Real>::build_graph(int nlaunch) {
     int blocks = 0, clusters = 0;
     size_t smem = 0;
     const int mode = advance_mode(cd_.pc.spec);
-    if (resident) TOMO_TRY(resident_clusters<Real>(plans_[plan_at_], plan_batch_[plan_at_], mode, &clusters));
-    else TOMO_TRY(advance_grid<Real>(blk_, mode, nitems_, num_sms_, &blocks, &smem));
+    if (resident) {
+        TOMO_TRY(resident_clusters<Real>(plans_[plan_at_], plan_batch_[plan_at_], mode, &clusters));
+        if (clusters < 1) return fail(TOMO_ECUDA, "a cluster of " + std::to_string(blk_.blocks) + " blocks does not fit the GPU");
+    } else TOMO_TRY(advance_grid<Real>(blk_, mode, nitems_, num_sms_, &blocks, &smem));
     cudaGraph_t graph;
     CUDA_TRY(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
     // one DFT pass per group of stage_group launches (and after the last launch):

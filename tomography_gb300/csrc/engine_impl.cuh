@@ -474,7 +474,8 @@ void make_resident(const ProblemClass& pc, const SolveLayout& lay, const Residen
 template <typename Real>
 int resident_choice(const ProblemClass& pc, const SolveLayout& lay, const Unpacked& u, ResidentPlan& p,
                     ResidentBatch& b);
-// Clusters of the batch that run at once.
+// Clusters of the batch that run at once; 0 where the GPU (or the part of it that this
+// process may use) has no room for one.
 template <typename Real>
 int resident_clusters(const ResidentPlan& p, const ResidentBatch& b, int mode, int* clusters);
 // Launches count solves from first on (around the end) on as many clusters; placed (may

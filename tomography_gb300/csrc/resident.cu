@@ -182,12 +182,15 @@ template <typename Real>
 int resident_clusters(const ResidentPlan& p, const ResidentBatch& b, int mode, int* clusters) {
     ResidentFn<Real> fn = resident_kernel_for<Real>(p.passes, mode, b.shape);
     if (!fn) return fail(TOMO_EINVAL, "no resident kernel for this grid");
+    *clusters = 0;
     CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemPerBlock));
     CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     cudaLaunchAttribute attr;
     cudaLaunchConfig_t c = cluster_config(p, b, 1, nullptr, &attr);
-    CUDA_TRY(cudaOccupancyMaxActiveClusters(clusters, fn, &c));
-    if (*clusters < 1) return fail(TOMO_ECUDA, "a cluster of " + std::to_string(p.blocks) + " blocks does not fit the GPU");
+    if (cudaOccupancyMaxActiveClusters(clusters, fn, &c) != cudaSuccess) {
+        cudaGetLastError();   // the answer to the question: no such cluster here
+        *clusters = 0;
+    }
     return TOMO_OK;
 }
 
@@ -220,6 +223,7 @@ int launch_resident(const ResidentPlan& p, const ResidentBatch& b, int mode, int
                     int nsolves, int first, int count, int nsteps, int* error, cudaStream_t st,
                     cudaEvent_t placed) {
     ResidentFn<Real> fn = resident_kernel_for<Real>(p.passes, mode, b.shape);
+    if (clusters < 1) return fail(TOMO_ECUDA, "a cluster of " + std::to_string(p.blocks) + " blocks does not fit the GPU");
     cudaLaunchAttribute attr[3];
     cudaLaunchConfig_t c = cluster_config(p, b, std::min(clusters, count), st, attr);
     // ahead of the DFT pass that runs beside it, whose blocks would hold up whole clusters
