@@ -7,11 +7,12 @@
 //     n_exc solves; a request may carry its own grid spec);
 //   * tomo_serve_step admits queued requests in FIFO order while their memory
 //     fits the HBM budget and descriptor slots are free, then advances EVERY
-//     admitted solve -- a request that fits the resident kernel by one launch
-//     of it, the others by up to four launches of the descriptor-driven
-//     wavefront kernel (solves of different requests, grid sizes and progress
-//     share the launches) -- and retires requests whose solves reached their last step
-//     (far field + misfit on the device, fitness to the host);
+//     admitted solve by about as many steps -- a request that fits the resident
+//     kernel by one launch of it, beside the other requests' launches, the others by
+//     launches of the descriptor-driven wavefront kernel that they share (solves
+//     of different requests, grid sizes and progress) -- and retires requests
+//     whose solves reached their last step (far field + misfit on the device,
+//     fitness to the host);
 //   * tomo_poll returns a finished request's fitness.
 // Each solve's arithmetic depends only on its own descriptor, so a result is
 // bit-identical whether the request ran alone or mixed with others.
@@ -30,6 +31,7 @@
 namespace tomo {
 
 constexpr int kServeSlots = 1 << 16;   // descriptor slots (solves in flight)
+constexpr int kServeStreams = 8;       // as many clusters of 16 blocks as run at once, and one
 
 enum ReqState { kQueued = 0, kRunning = 1, kDone = 2, kCancelled = 3, kFailed = 4 };
 
@@ -67,6 +69,10 @@ struct ServeRequest {
 template <typename Real>
 struct ServeStateT {
     DevBuf descs, items;
+    // requests on the resident kernel run on these streams, beside each other and beside the
+    // wavefront launches; every serving step joins them
+    cudaStream_t side[kServeStreams] = {};
+    cudaEvent_t begun = nullptr, ended[kServeStreams] = {};
     DevBuf lost;   // error words of the resident kernel, a request's at its first slot
     std::vector<SolveDesc<Real>> hdescs;
     std::vector<char> used;
@@ -81,6 +87,22 @@ struct ServeStateT {
     int hi_slot = 0;   // one past the highest slot ever used
     Blocking blk{0, 0, 0};   // blocking of the serving loop, fixed at the first serving step
     int cmax = 0, fmax = 1;   // largest NTFF contour and most frequencies among the running requests
+
+    int create_streams() {
+        CUDA_TRY(cudaEventCreateWithFlags(&begun, cudaEventDisableTiming));
+        for (int i = 0; i < kServeStreams; ++i) {
+            CUDA_TRY(cudaStreamCreateWithFlags(&side[i], cudaStreamNonBlocking));
+            CUDA_TRY(cudaEventCreateWithFlags(&ended[i], cudaEventDisableTiming));
+        }
+        return TOMO_OK;
+    }
+    ~ServeStateT() {
+        for (cudaEvent_t e : ended)
+            if (e) cudaEventDestroy(e);
+        if (begun) cudaEventDestroy(begun);
+        for (cudaStream_t s : side)
+            if (s) cudaStreamDestroy(s);
+    }
 
     int find_range(int n) {
         int run = 0;
@@ -105,6 +127,7 @@ static ServeStateT<Real>* serve_state(ServeStateT<Real>*& s, int* rc) {
     if (*rc == TOMO_OK) *rc = st->lost.ensure(sizeof(int) * kServeSlots);
     if (*rc == TOMO_OK && cudaMemset(st->lost.p, 0, sizeof(int) * kServeSlots) != cudaSuccess)
         *rc = fail(TOMO_ECUDA, "cudaMemset of the serving error words failed");
+    if (*rc == TOMO_OK) *rc = st->create_streams();
     if (*rc) {
         delete st;
         return nullptr;
@@ -394,38 +417,67 @@ int EngineT<Real>::serve_step(int* n_active) {
         CUDA_TRY(cudaStreamSynchronize(stream_));
         st->items_dirty = false;
     }
-    // 3. advance everything admitted.  Requests on the resident kernel: one launch
-    // of up to kServeSteps steps each (the kernel ends at a solve's last step).
-    // The others together: as many wavefront launches as the one closest to its
-    // end still needs, at most kLaunchesPerStep, so that no request runs past its
-    // last step.  The host synchronises after the launches, and once more for what they retire.
-    constexpr int kServeSteps = 128, kLaunchesPerStep = 4;
-    const int mode = advance_mode(cd_.pc.spec);
-    int running = 0, nl = st->nitems > 0 ? kLaunchesPerStep : 0;
-    bool resident = false;
+    // 3. advance everything admitted.  The resident kernel's requests take one launch each, on
+    // streams of their own (sixteen requests of one 200^2 solve: 37 ms one after another,
+    // 8.5 ms so); the others share wavefront launches, until the one closest to its end
+    // has finished, so that none runs past its last step.  Beside kServeSteps resident steps
+    // go as many wavefront steps as keep the resident requests' part of the GPU to about a
+    // sixth, but a third of the steps at most: there the wavefront requests advance no slower
+    // than with all requests in the wavefront kernel, where a step of the small ones costs
+    // three times as much (600^2 beside six requests of four 200^2 solves: 48 ms there, 45 ms
+    // here, 230 ms with four launches whatever runs beside).  The host
+    // synchronises after the launches, and once more for what they retire.
+    constexpr int kServeSteps = 128;
+    constexpr double kSweepCells = sizeof(Real) == 4 ? 150e3 : 15e3;   // cells a microsecond
+    const int mode = advance_mode(cd_.pc.spec), T = st->blk.T;
+    bool resident = false, streaming = false;
+    double chip = 0, sweep = 0;   // about the whole GPU's microseconds of a step
     for (auto& kv : st->reqs) {
-        ServeRequest<Real>& r = *kv.second;
+        const ServeRequest<Real>& r = *kv.second;
         if (!r.advances()) continue;
-        const ProblemClass& pc = r.cd->pc;
-        if (!r.resident) {
-            nl = std::min(nl, (pc.S - r.steps_done + st->blk.T - 1) / st->blk.T);
-            continue;
-        }
-        SolveDesc<Real>* const d = st->descs.template as<SolveDesc<Real>>() + r.first;
-        const int steps = std::min(kServeSteps, r.plan.levels);
-        TOMO_TRY(launch_resident<Real>(r.plan, r.batch, mode, r.clusters, d, r.nsolves, 0, r.nsolves, steps,
-                                       st->lost.template as<int>() + r.first, stream_));
-        resident = true;
-        if (dft_contour(pc) > 0)
-            launch_dft<Real>(d, r.nsolves, dft_contour(pc), pc.nfreq, steps, -1, steps, 1, stream_);
-        bump_kernel<Real><<<(r.nsolves + 127) / 128, 128, 0, stream_>>>(d, r.nsolves, steps, nullptr, 1, 0, r.nsolves);
-        r.steps_done += steps;
+        (r.resident ? resident : streaming) = true;
+        if (r.resident) chip += (double)r.nsolves * r.plan.blocks / num_sms_ * (0.9 + r.batch.cost);
+        else sweep += (double)r.nsolves * r.cd->pc.nx * r.cd->pc.ny / kSweepCells;
     }
-    for (int l = 0; l < nl; ++l)
-        launch_advance<Real>(st->blk, mode, st->blocks, st->smem, st->descs.template as<SolveDesc<Real>>(),
-                             st->items.template as<WorkItem>(), st->nitems, st->hi_slot, d_counter_.as<int>(), st->cmax,
-                             st->fmax, stream_);
-    CUDA_TRY(cudaGetLastError());
+    const double even = sweep > 0 ? 6 * kServeSteps * chip / sweep : 0;
+    int nl = ((int)std::max(kServeSteps / 16.0, std::min(kServeSteps / 3.0, even)) + T - 1) / T;
+    for (auto& kv : st->reqs) {
+        const ServeRequest<Real>& r = *kv.second;
+        if (r.advances() && !r.resident) nl = std::min(nl, (r.cd->pc.S - r.steps_done + T - 1) / T);
+    }
+    auto launch = [&]() -> int {
+        if (resident) CUDA_TRY(cudaEventRecord(st->begun, stream_));
+        int turn = 0;
+        for (auto& kv : st->reqs) {
+            ServeRequest<Real>& r = *kv.second;
+            if (!r.advances() || !r.resident) continue;
+            const cudaStream_t side = st->side[turn % kServeStreams];
+            if (turn++ < kServeStreams) CUDA_TRY(cudaStreamWaitEvent(side, st->begun, 0));
+            const ProblemClass& pc = r.cd->pc;
+            SolveDesc<Real>* const d = st->descs.template as<SolveDesc<Real>>() + r.first;
+            const int steps = std::min(kServeSteps, r.plan.levels);
+            TOMO_TRY(launch_resident<Real>(r.plan, r.batch, mode, r.clusters, d, r.nsolves, 0, r.nsolves, steps,
+                                           st->lost.template as<int>() + r.first, side));
+            if (dft_contour(pc) > 0)
+                launch_dft<Real>(d, r.nsolves, dft_contour(pc), pc.nfreq, steps, -1, steps, 1, side);
+            bump_kernel<Real><<<(r.nsolves + 127) / 128, 128, 0, side>>>(d, r.nsolves, steps, nullptr, 1, 0, r.nsolves);
+            r.steps_done += steps;
+        }
+        for (int l = 0; streaming && l < nl; ++l)
+            launch_advance<Real>(st->blk, mode, st->blocks, st->smem, st->descs.template as<SolveDesc<Real>>(),
+                                 st->items.template as<WorkItem>(), st->nitems, st->hi_slot, d_counter_.as<int>(),
+                                 st->cmax, st->fmax, stream_);
+        CUDA_TRY(cudaGetLastError());
+        for (int i = 0; i < std::min(turn, kServeStreams); ++i) {
+            CUDA_TRY(cudaEventRecord(st->ended[i], st->side[i]));
+            CUDA_TRY(cudaStreamWaitEvent(stream_, st->ended[i], 0));
+        }
+        return TOMO_OK;
+    };
+    if (const int failed = launch()) {
+        for (cudaStream_t side : st->side) cudaStreamSynchronize(side);   // nothing runs on unjoined
+        return failed;
+    }
     std::vector<int> lost(resident ? st->hi_slot : 0);
     if (resident) {
         CUDA_TRY(cudaMemcpyAsync(lost.data(), st->lost.p, sizeof(int) * lost.size(), cudaMemcpyDeviceToHost, stream_));
@@ -433,6 +485,7 @@ int EngineT<Real>::serve_step(int* n_active) {
     }
     // a request whose halo row did not arrive has no result: it fails, and returns what it holds
     bool failed = false;
+    int running = 0;
     for (auto& kv : st->reqs) {
         ServeRequest<Real>& r = *kv.second;
         if (!r.advances() || !r.resident || !lost[r.first]) continue;
@@ -445,7 +498,7 @@ int EngineT<Real>::serve_step(int* n_active) {
     for (auto& kv : st->reqs) {
         ServeRequest<Real>& r = *kv.second;
         if (!r.advances()) continue;
-        if (!r.resident) r.steps_done += nl * st->blk.T;
+        if (!r.resident) r.steps_done += nl * T;
         if (r.steps_done >= r.cd->pc.S) TOMO_TRY(retire(st, r, stream_, true));
         else ++running;
     }
