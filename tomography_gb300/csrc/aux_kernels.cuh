@@ -205,9 +205,10 @@ __global__ void __launch_bounds__(256) farfield_kernel(const Real* __restrict__ 
 // product), the errors and their errors are added up beside the values, and a
 // chunk's sums join in FP64.  Against exact sums of 1000 to 240000 samples the
 // relative error is 0.8e-16 to 1.7e-16 rms, the FP64 sums' 1.1e-16 to 1.9e-16.
-// (Without the errors' errors: 1.9e-16 to 2.5e-16, in 87 us.)  A chunk whose sum
+// (Without the errors' errors: 1.9e-16 to 2.5e-16, in 87 us.)  A chunk's sum that
 // is outside [2^-70, 2^100] -- where products would lose bits to underflow or
-// overflow -- or not finite is done in FP64.
+// overflow -- or not finite is done in FP64, num and den each for itself: only the
+// first candidate's solves take den, and num must not depend on it.
 constexpr int kMisfitChunk = 8192;
 inline int misfit_chunks(size_t n_per_solve) { return (int)((n_per_solve + kMisfitChunk - 1) / kMisfitChunk); }
 
@@ -288,16 +289,19 @@ __device__ __forceinline__ double misfit_join(double v, double* part) {
     return a;
 }
 
-// One chunk in FP64: the general form.
+// One chunk in FP64, the general form: num and den, either of which may be null.
 template <typename Real>
 __device__ inline void misfit_chunk_fp64(const Real* tr, const float* tg, int n, double* part, double* num, double* den,
                                          int* nonfinite) {
     double a = 0, b = 0;
     int bad = 0;
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const double sv = (double)tr[i], tv = (double)tg[i];
-        if (!isfinite(sv)) bad = 1;
-        a += (sv - tv) * (sv - tv);
+        const double tv = (double)tg[i];
+        if (num) {
+            const double sv = (double)tr[i];
+            if (!isfinite(sv)) bad = 1;
+            a += (sv - tv) * (sv - tv);
+        }
         if (den) b += tv * tv;
     }
     for (int o = 16; o > 0; o >>= 1) {
@@ -306,13 +310,16 @@ __device__ inline void misfit_chunk_fp64(const Real* tr, const float* tg, int n,
     }
     bad = __any_sync(0xffffffffu, bad);
     if (bad && (threadIdx.x & 31) == 0) atomicOr(nonfinite, 1);
-    *num = misfit_join(a, part);
+    if (num) *num = misfit_join(a, part);
     if (den) *den = misfit_join(b, part);
 }
 
-// One chunk of FP32 traces with split sums; false when its sums ask for FP64.
-__device__ inline bool misfit_chunk_split(const float* tr, const float* tg, int n, bool aligned, double* part,
-                                          double* num, double* den) {
+// One chunk of FP32 traces with split sums; which of them ask for FP64.
+struct MisfitRedo {
+    bool num, den;   // the same in every thread
+};
+__device__ inline MisfitRedo misfit_chunk_split(const float* tr, const float* tg, int n, bool aligned, double* part,
+                                                double* num, double* den) {
     SplitSum d, t;
     // the same samples to the same threads whatever the alignment
     auto four = [&](const float* p, int i) {
@@ -337,8 +344,9 @@ __device__ inline bool misfit_chunk_split(const float* tr, const float* tg, int 
     float(*const parts)[3] = reinterpret_cast<float(*)[3]>(part);
     *num = d.block_total(parts);
     if (den) *den = t.block_total(parts);
-    auto safe = [](double v) { return v >= 0x1p-70 && v <= 0x1p100; };
-    return __syncthreads_and(threadIdx.x != 0 || (safe(*num) && (!den || safe(*den))));
+    auto redo = [](double v) { return __syncthreads_or(threadIdx.x == 0 && !(v >= 0x1p-70 && v <= 0x1p100)) != 0; };
+    const bool redo_num = redo(*num);
+    return {redo_num, den && redo(*den)};
 }
 
 // num [nsolves][parts] and den [n_tx][parts]: gridDim.y = parts blocks per solve
@@ -359,12 +367,13 @@ __global__ void __launch_bounds__(256)
         const Real* tr = traces + (size_t)s * tr_stride + at;
         const float* tg = target + (size_t)tx * n_per_solve + at;
         double cn = 0, cd = 0;
-        bool done = false;
+        MisfitRedo redo{true, with_den};
         if constexpr (sizeof(Real) == 4) {
             const bool aligned = (((size_t)tr | (size_t)tg) & 15) == 0;
-            done = misfit_chunk_split(tr, tg, n, aligned, part, &cn, with_den ? &cd : nullptr);
+            redo = misfit_chunk_split(tr, tg, n, aligned, part, &cn, with_den ? &cd : nullptr);
         }
-        if (!done) misfit_chunk_fp64<Real>(tr, tg, n, part, &cn, with_den ? &cd : nullptr, nonfinite);
+        if (redo.num || redo.den)
+            misfit_chunk_fp64<Real>(tr, tg, n, part, redo.num ? &cn : nullptr, redo.den ? &cd : nullptr, nonfinite);
         a += cn;
         b += cd;
     }
