@@ -46,3 +46,21 @@ def test_places_in_the_batch(tomo, quiet):
             assert got.setdefault(c, fit) == fit, (quiet, c, order)
     for c in range(3):
         assert _misfit(tomo, traces[c:c + 1], target)[0] == got[c]
+
+
+@pytest.mark.parametrize("chunks,more", [(65535, 0), (65535, 1), (65536, 0), (65536, 1)])
+def test_longest_solves(tomo, chunks, more):
+    """Around the most chunks that one solve spreads over a grid: sums that are exact."""
+    import ctypes as C
+
+    import torch
+
+    m = chunks * CHUNK + more
+    target = torch.ones(m, dtype=torch.float32, device="cuda")
+    traces = torch.full((m,), 1.5, dtype=torch.float32, device="cuda")
+    fit = torch.full((1,), float("nan"), dtype=torch.float64, device="cuda")
+    lib = tomo.library()
+    rc = lib.tomo_trace_misfit_static(C.c_void_p(traces.data_ptr()), C.c_void_p(target.data_ptr()), 1, 1, m,
+                                      C.c_void_p(fit.data_ptr()), C.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert rc == 0, lib.tomo_last_error()
+    assert fit.item() == -0.25

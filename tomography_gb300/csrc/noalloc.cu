@@ -90,9 +90,10 @@ extern "C" int tomo_trace_misfit_static(const float* traces, const float* target
         e = cudaMemsetAsync(flag, 0, sizeof(int) * 4, st);   // the flag must start at zero every call
         if (e != cudaSuccess) return fail(TOMO_ECUDA, std::string("cudaMemsetAsync: ") + cudaGetErrorString(e));
         // a block for every chunk of a solve where the scratch holds their sums (the first
-        // half the solves', the second the transmitters'): a few solves then fill the GPU
+        // half the solves', the second the transmitters') and a grid may have as many
+        // rows: a few solves then fill the GPU
         const size_t chunks = (size_t)tomo::misfit_chunks(n_per_solve);
-        const int parts = chunks * n_cand * n_tx <= tomo::kNoAllocMaxSolves ? (int)chunks : 1;
+        const int parts = chunks <= 65535 && chunks * n_cand * n_tx <= tomo::kNoAllocMaxSolves ? (int)chunks : 1;
         double* const den = partials + tomo::kNoAllocMaxSolves;
         tomo::trace_partials_kernel<float><<<dim3(nsolves, parts), 256, 0, st>>>(traces, n_per_solve, target,
                                                                                  (int)n_per_solve, (int)n_tx, partials,
