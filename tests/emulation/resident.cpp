@@ -62,7 +62,7 @@ static int launch(std::vector<SolveDesc<Real>> descs, int blocks, std::function<
     const SolveDesc<Real>& d = descs[0];
     int tall = 0, error = 0;
     for (int b = 0; b < blocks; ++b) tall = std::max(tall, d.ys[b + 1] - d.ys[b]);
-    const int threads = 32 * ((tall + kShare - 1) / kShare);
+    const int threads = 32 * resident_warps(tall, kShare, d.nrx);
     HostCluster c;
     cluster = &c;
     c.blocks.resize(blocks);

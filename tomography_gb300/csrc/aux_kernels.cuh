@@ -344,9 +344,11 @@ __device__ inline MisfitRedo misfit_chunk_split(const float* tr, const float* tg
     float(*const parts)[3] = reinterpret_cast<float(*)[3]>(part);
     *num = d.block_total(parts);
     if (den) *den = t.block_total(parts);
-    auto redo = [](double v) { return __syncthreads_or(threadIdx.x == 0 && !(v >= 0x1p-70 && v <= 0x1p100)) != 0; };
-    const bool redo_num = redo(*num);
-    return {redo_num, den && redo(*den)};
+    __shared__ MisfitRedo redo;
+    auto outside = [](double v) { return !(v >= 0x1p-70 && v <= 0x1p100); };
+    if (threadIdx.x == 0) redo = {outside(*num), den && outside(*den)};
+    __syncthreads();
+    return redo;
 }
 
 // num [nsolves][parts] and den [n_tx][parts]: gridDim.y = parts blocks per solve

@@ -118,7 +118,7 @@ static bool batch_on(const ProblemClass& pc, const ResidentPlan& p, const Reside
         else if (!cut_slabs<Real>(pc, p, shape, m, cost, ys, b.cost)) return false;
         int tall = 0;
         for (int k = 0; k < p.blocks; ++k) tall = std::max(tall, ys[k + 1] - ys[k]);
-        b.warps = std::max(b.warps, (tall + shape.share - 1) / shape.share);
+        b.warps = std::max(b.warps, resident_warps(tall, shape.share, pc.nrx));
         for (int k = 0; k < p.blocks; ++k)
             b.smem = std::max(b.smem, resident_layout<Real>(pc.nx, pc.ny, pc.nc, pc.nmat, ref, p.passes, shape.share, ys[k],
                                                             ys[k + 1], tall, m[0], m[1], m[2], m[3], d)
