@@ -8,7 +8,9 @@ steps, FP32 fields), seeded synthetic candidates and target, through the C ABI.
           stream around set-up + time loop + far field + misfit; inputs resident)
   e2e   : evals/s of the same C-ABI call timed on the host with host buffers
           (H2D of the candidate parameters, D2H of the fitness inside)
-  roofline : the advance kernel, algorithmic 48 B per FP32 cell-update
+  roofline : the kernel of the time loop: the resident kernel by its arithmetic (12
+          operations a cell-update against the FP32 units), the wavefront kernel by
+          its algorithmic 48 B per FP32 cell-update against HBM
   cpu_baseline : the oracle's FP32 port of the reference CPU solver, one
           candidate (16 solves) on all host cores
 
@@ -36,6 +38,7 @@ METRIC = "PSO fitness evals/s"
 CONFIG_INDEX = 1
 N_CAND = 256
 BYTES_PER_CELL_UPDATE = 48.0   # FP32: Ez, Hx, Hy, Jp read+write + 4 per-cell coefficients
+FLOPS_PER_CELL_UPDATE = 12.0   # Hx and Hy: 3 each; Ez: 6 (the Debye current's 6 more, inside the tissue, left out)
 
 
 def _rank_info():
@@ -313,21 +316,31 @@ def run_ours(args) -> None:
     value = units / tot_dev
     e2e = units / tot_wall
 
-    # roofline of the advance kernel (average launch over the timed region)
+    # roofline of the time loop's kernel (average launch over the timed region)
     launches = st["launches"]
     cells_per_launch = st["cell_updates"] / launches   # solves * nx * ny * T (average over launches)
     launch_s = (sum(adv_ms) / len(adv_ms)) / 1e3 / launches
     achieved = BYTES_PER_CELL_UPDATE * cells_per_launch / launch_s / 1e9
     peaks = _peaks()
-    tr = _profile_traffic(st["steps_per_launch"], st["cols_per_lane"], st.get("min_blocks_per_sm", 2))
-    roofline = {"bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
-                "frac": achieved / peaks["hbm_gbs"], "peak_source": peaks["source"],
-                "traffic": (tr * cells_per_launch) if tr is not None else None,
-                "algorithmic_bytes_per_launch": BYTES_PER_CELL_UPDATE * cells_per_launch,
-                "kernel": ("fdtd_resident_kernel<float>, up to %d steps a launch" % st["steps_per_launch"]
-                           if st.get("min_blocks_per_sm", 2) == 1 else
-                           "fdtd_advance_kernel<float,%d,%d> (min %d blocks/SM)" % (
-                               st["steps_per_launch"], st["cols_per_lane"], st.get("min_blocks_per_sm", 2)))}
+    if st.get("min_blocks_per_sm", 2) == 1:
+        # the resident kernel: the fields stay on the chip, so that its floor is arithmetic
+        sms = torch.cuda.get_device_properties(dev).multi_processor_count
+        mhz = (clocks or {}).get("sm_max_mhz") or 2070.0
+        tflops = FLOPS_PER_CELL_UPDATE * cells_per_launch / launch_s / 1e12
+        peak = sms * 128 * 2 * mhz / 1e6
+        roofline = {"bound": "fp32", "achieved": tflops, "peak": peak, "unit": "TFLOP/s", "frac": tflops / peak,
+                    "peak_source": "%d SMs x 128 lanes x 2 at %g MHz" % (sms, mhz), "traffic": None,
+                    "algorithmic_bytes_per_launch": BYTES_PER_CELL_UPDATE * cells_per_launch,
+                    "algorithmic_gbs": achieved,
+                    "kernel": "fdtd_resident_kernel<float>, up to %d steps a launch" % st["steps_per_launch"]}
+    else:
+        tr = _profile_traffic(st["steps_per_launch"], st["cols_per_lane"], st.get("min_blocks_per_sm", 2))
+        roofline = {"bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
+                    "frac": achieved / peaks["hbm_gbs"], "peak_source": peaks["source"],
+                    "traffic": (tr * cells_per_launch) if tr is not None else None,
+                    "algorithmic_bytes_per_launch": BYTES_PER_CELL_UPDATE * cells_per_launch,
+                    "kernel": "fdtd_advance_kernel<float,%d,%d> (min %d blocks/SM)" % (
+                        st["steps_per_launch"], st["cols_per_lane"], st.get("min_blocks_per_sm", 2))}
     gcells = st["cell_updates"] * world * args.steps / tot_dev / 1e9
 
     extra = {}

@@ -116,14 +116,16 @@ typedef struct tomo_stats {
     double cell_updates;      /* Ez cells x steps advanced in the last batch                */
     int64_t launches;         /* advance-kernel launches in the last batch                  */
     int64_t kernels;          /* all kernels launched in the last batch                     */
-    int32_t steps_per_launch; /* T used                                                      */
-    int32_t cols_per_lane;    /* COLS used                                                   */
+    int32_t steps_per_launch; /* T used; on the resident kernel the most steps of a launch   */
+    int32_t cols_per_lane;    /* COLS used; on the resident kernel the columns of 16 bytes   */
     int64_t h2d_bytes, d2h_bytes;  /* host<->device bytes of the last batch                  */
     double tune_ms;           /* device time the autotuner spent in the last call (0 when
                                  the (T, COLS) choice for this batch size was cached)     */
     int32_t tuned_configs;    /* blockings the autotuner timed in the last call            */
     int32_t min_blocks_per_sm;/* register budget of the advance kernel used (2: 255 regs,
-                                 3: 168, 4: 128 per thread)                               */
+                                 3: 168, 4: 128 per thread); 1: the resident kernel ran.
+                                 Its steps_per_launch and cols_per_lane are no blocking
+                                 that a spec can ask for: leave the spec's at 0           */
     /* serving loop, as of the end of the last tomo_serve_step */
     uint64_t serve_bytes_in_use;  /* device bytes held by admitted requests               */
     int32_t serve_running;        /* admitted requests still advancing                    */

@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(256) farfield_kernel(const Real* __restrict__ 
 // chunk has a block of its own: the result does not depend on the batch.
 //
 // FP64 sums were bound by the FP64 units (two lanes a clock and SM, five
-// operations a sample: 596 us for 49 M samples, 5% of HBM; now 113 us, bound by
+// operations a sample: 596 us for 49 M samples, 5% of HBM; now 97 us, bound by
 // some 40 FP32 operations a sample).  FP32 traces are summed in FP32 without
 // their rounding errors instead: the difference, its square and every addition
 // are split into a value and its exact error (Knuth's two-sum, an fma for a

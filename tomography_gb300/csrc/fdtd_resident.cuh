@@ -26,20 +26,24 @@
 // A step ends with one block barrier; blocks wait for each other's halo rows
 // only.  Then the threads of a block sample the step, the warps with the fewest
 // rows first: the receivers to the traces and the NTFF contour to the staging buffer.
+// A solve ends with a cluster barrier, behind the write-back: no block may overwrite
+// its rows, or end, before its neighbours have taken the last one.
 //
-// What bounds it.  Latency and issue of few warps: a block with materials issues on
-// 30% of its slots and uses the shared memory pipe at 47%, and a step cannot be
-// shorter than the slowest warp's passes (400^2, cluster of 16: about 500 cycles
+// What bounds it.  Latency and issue of few warps: 400^2 with its breast phantom on 16
+// blocks issues on 36% of its slots and uses the shared memory pipe at 49%, and a step
+// cannot be shorter than the slowest warp's passes (about 500 cycles
 // of halo wait, 900 of edge pass, 500 to 1200 a pass, 400 of sampling).  So a
 // warp holds as few rows as the registers allow: with two rows, 16 warps of 128
-// registers (12 of 168 in FP64 and where 24 rows a block are enough) a step takes
-//   400^2  2.98 us, against 3.60 with four rows and 8 warps of 255 registers,
-//   200^2  1.69 us, against 2.53;   333 x 251  2.00 us, against 2.91,
-//   FP64 200^2  14.1 us, against 25.0 (bound by the FP64 units, two lanes a clock).
+// registers (12 of 168 in FP64 and where 24 rows a block are enough) a step of one
+// solve takes, with its share of the launches and the DFT,
+//   400^2  2.5 us, against 3.6 with four rows and 8 warps of 255 registers,
+//   200^2  1.9 us, against 2.5;   333 x 251  2.1 us, against 2.9,
+//   FP64 200^2  15 us, against 25 (of which the FP64 pipe is busy 10.7: two lanes a
+//   clock and 18 instructions a cell, and the passes' latency beside it).
 // Three rows (12 warps) spill and run at 3.64 us on 400^2.  Ez of a warp's own
 // rows kept in registers too: 4.19 us, the four-row passes lose the room to load ahead.
 // Four rows stay where two would not hold the grid: 512 columns, tall narrow grids.
-// The wavefront kernel took 14.3 ms for a 200^2 forward of 1000 steps, this one 2.2.
+// The wavefront kernel took 14.3 ms for a 200^2 forward of 1000 steps, this one 2.1.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>

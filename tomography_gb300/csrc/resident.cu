@@ -7,7 +7,12 @@ namespace tomo {
 // The shapes in the order of their speed: the first that holds a batch takes it.  Two
 // rows a warp beat four wherever both hold the slabs (400^2: 2.98 against 3.60 us a step);
 // 12 warps leave 168 registers, 16 leave 128 and some spills (384 rows of 400: 2.89
-// against 3.17 us).
+// against 3.17 us).  Which of them are compiled for a number of inner passes follows the
+// grids in use, not a limit of the kernel: two rows on 16 warps and 16 blocks hold 512
+// rows, any square of one to three passes (up to 415 columns); four rows are there for
+// what two do not hold, tall grids of one pass (768 rows) and four passes, where the
+// fields of two rows take 80 of 16 warps' 128 registers.  The reference modes' problem
+// (401^2) takes three passes, FP64 one to three.  Other grids take the wavefront kernel.
 static constexpr ResidentShape kShapes[] = {{2, 12}, {2, 16}, {4, 12}, {4, 8}};
 
 template <typename Real>
