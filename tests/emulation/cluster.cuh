@@ -53,8 +53,8 @@ inline HostCluster* cluster = nullptr;
 inline double host_seconds() {
     return std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch()).count();
 }
-// The kernel waits for a row for 4e9 clocks: one second.
-inline long long clock64() { return (long long)(host_seconds() * 4e9); }
+// The kernel waits for a row for 4e9 clocks: two seconds.
+inline long long clock64() { return (long long)(host_seconds() * 2e9); }
 
 namespace tomo {
 

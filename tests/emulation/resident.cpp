@@ -117,7 +117,7 @@ int main(int argc, char** argv) {
     auto delay = [&](int to, int index) {
         if (what == "ends") return 0.0;
         if (what == "late") return to == 0 ? 0.1 : 0.0;
-        return to == 1 && index == 1 ? (what == "lost" ? -1.0 : 1.3) : 0.0;
+        return to == 1 && index == 1 ? (what == "lost" ? -1.0 : 2.6) : 0.0;
     };
     const int error = launch(both, blocks, delay, &faults);
     if (what == "ends") {
