@@ -560,15 +560,21 @@ inline void append_items(std::vector<WorkItem>& items, int first, int nsolves, i
             }
         }
     const bool aligned = cols == 1 || (2 * T) % cols == 0;   // then every wide boundary stays = T
+    // A vertical face's sample takes Ez of the column to its right, which the last level has
+    // for a strip's owned columns alone: no strip ends with a face column.
+    auto strip_end = [&](int x, int end) {
+        const int x1 = std::min(x + W1, end);
+        return d >= 0 && x1 < ncol && (x1 - 1 == d || x1 - 1 == nx - d - 1) ? x1 - 1 : x1;
+    };
     if (cols == 1 || !aligned || best < 0) {
-        const int n = (ncol + W1 - 1) / W1;
-        for (int q = 0; q < n; ++q) {
-            const WorkItem w{0, q * W1, std::min((q + 1) * W1, ncol), cols > 1 ? 1 : 0, 0, ny + 1};
-            (q == 0 || q == n - 1 ? edge : mid).push_back(w);
+        for (int x = 0, x1; x < ncol; x = x1) {
+            x1 = strip_end(x, ncol);
+            const WorkItem w{0, x, x1, cols > 1 ? 1 : 0, 0, ny + 1};
+            (x == 0 || x1 == ncol ? edge : mid).push_back(w);
         }
     } else {
-        for (int x = 0; x < a; x += W1) edge.push_back({0, x, std::min(x + W1, a), 1, 0, ny + 1});
-        for (int x = b; x < ncol; x += W1) edge.push_back({0, x, std::min(x + W1, ncol), 1, 0, ny + 1});
+        for (int x = 0, x1; x < a; x = x1) edge.push_back({0, x, x1 = strip_end(x, a), 1, 0, ny + 1});
+        for (int x = b, x1; x < ncol; x = x1) edge.push_back({0, x, x1 = strip_end(x, ncol), 1, 0, ny + 1});
         for (int x = a; x < b; x += W2) mid.push_back({0, x, std::min(x + W2, b), 0, 0, ny + 1});
     }
     // row segments: [0, ny] cut into nseg nearly equal ranges
@@ -627,6 +633,7 @@ inline int validate_items(const std::vector<WorkItem>& items, size_t first_item,
             bad = bad || xs <= ncpml || xs + P - 1 >= nx - ncpml;
             if (d >= 0) bad = bad || (d >= xs && d < xs + P) || (nx - d - 1 >= xs && nx - d - 1 < xs + P);
         }
+        if (d >= 0 && w.x1 <= nx) bad = bad || w.x1 - 1 == d || w.x1 - 1 == nx - d - 1;
         if (bad)
             return fail(TOMO_ECUDA, "internal error: work item (" + std::to_string(w.x0) + ", " + std::to_string(w.x1) +
                                         ") invalid for nx " + std::to_string(nx));
